@@ -238,18 +238,21 @@ typedef struct {
   int precond;
   uint32_t schwarz_domain;
   int precision;
-  int pcg_mode;            /* 0: two fused kernels per iteration (rows, domains) at full
-                                 occupancy, replayed as CUDA graphs (default);
+  int pcg_mode;            /* 0, 2: one cooperative launch per linear solve, the system resident in
+                                 the SMs' shared memory; systems too large for it (beyond about
+                                 64 Schwarz domains or 2 000 vertices per SM) and scenes with a
+                                 pcg_variant run two fused kernels per iteration (rows, domains)
+                                 at full occupancy, replayed as CUDA graphs;
                               1: one launch per PCG kernel, replayed as CUDA graphs (single
-                                 scenes only);
-                              2: one cooperative persistent launch per linear solve */
+                                 scenes only) */
   int factor_storage;      /* Schwarz factor tiles: 0 = by precision (FP32 tiles with
                               MGUSO_PRECISION_FP32, FP16 tiles scaled per domain with MIXED),
                               1 = FP32 tiles, 2 = FP16 tiles */
   uint32_t schwarz_levels; /* 1 (or 0): one-level Schwarz (SchwarzCpu, linsolve.rs:463-520);
                               2: two-level Galerkin Schwarz (SchwarzMlCpu, linsolve.rs:534-836) */
-  int pcg_variant;         /* kernels of the fused PCG (pcg_mode 0): 0 = chosen by the autotuner
-                              at the scene's first solve (cached per system size); v in 1..24
+  int pcg_variant;         /* 0 = the resident PCG where it fits, else the fused kernels chosen by
+                              an autotuner at the scene's first fused solve (cached per system
+                              size); v in 1..24 runs the fused PCG (pcg_mode 0, 2) and
                               fixes the rows kernel (v - 1) / 6 (0, 1, 2: 2, 1 or 4 lanes per
                               block row over the BSR; 3: one lane per row over a sliced-ELL copy)
                               and the Schwarz domain kernel (v - 1) % 6 (0: one warp per domain,
@@ -454,10 +457,11 @@ int mguso_scene_profile(mguso_scene* s, int reps, float* us4, double* bytes4);
  * SpMV, p.Ap), domain kernel (x/r update, preconditioner apply, r.r and r.z)}; bytes2 =
  * their algorithmic bytes per launch. Clobbers the PCG scratch (not the state). */
 int mguso_scene_profile_pcg(mguso_scene* s, int iters, float* us2, double* bytes2);
-/* The fused PCG kernels in use, as the autotuner (or pcg_variant) chose them: out2 = {rows
+/* The fused PCG kernels that a fused solve or mguso_scene_profile_pcg runs, as the autotuner (or
+ * pcg_variant) chose them: out2 = {rows
  * kernel: 0 two lanes per block row, 1 one, 2 four, 3 sliced ELL; domain kernel: 0 one warp per domain and
  * four domains per CTA, 1/2/3 three warps per domain and 1/2/4 domains per CTA}; -1 before
- * the scene's first solve. */
+ * the scene's first fused solve or profile. */
 int mguso_scene_pcg_kernels(mguso_scene* s, int* out2);
 
 /* The self-intersection scan behind mguso_step_stats.penetration_free

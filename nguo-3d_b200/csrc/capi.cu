@@ -280,6 +280,7 @@ int mguso_linear_solve(mguso_linear_solver* s, const mguso_csr* a, const float* 
     s->csr_row_ptr.assign(a->row_ptr, a->row_ptr + a->n + 1);
     s->csr_col.assign(a->col_idx, a->col_idx + nnz);
     s->generation++;
+    s->rs_ready = false;
     if (s->precond == MGUSO_PRECOND_SCHWARZ) {
       s->schwarz = std::make_unique<mguso_schwarz>();
       s->schwarz->a = s->bsr.get();

@@ -79,6 +79,7 @@ struct mguso_schwarz {
   mg::DevBuf<uint32_t> dom_verts;  // nb
   mg::DevBuf<uint32_t> dom_of;     // nb
   mg::DevBuf<uint32_t> loc;        // nb: local index of a vertex inside its domain
+  mg::DevBuf<uint32_t> vpos;       // nb: a vertex's place in dom_verts
   mg::DevBuf<uint64_t> fac_off;    // ndom + 1 (float offsets, 4-float aligned)
   mg::DevBuf<float> fac;           // W = L^-1 per domain, swizzled 32x32 FP32 tiles
   uint64_t fac_floats = 0;         // elements of the tile storage
@@ -186,10 +187,60 @@ struct PcgInstResult {
   uint32_t iters, status, done, pad;
 };
 
+// ---- resident PCG (pcg_resident.cu) ---------------------------------------------------
+// The system A + C and its preconditioner, all device pointers. Schwarz: domains are runs of
+// `dom_verts` (a vertex's place in it is its position, vpos), block-diagonal domains of an
+// instance after its others; block Jacobi: position = vertex.
+struct RsSystem {
+  const uint32_t *rp, *col;
+  const float* val;
+  const uint32_t *crp, *ccol;  // blocks outside the pattern (null: none)
+  const float* cval;
+  const uint32_t *dom_start, *dom_verts, *vpos;
+  const uint64_t* fac_off;
+  const void* fac;         // float or __half tiles
+  const float* fac_scale;  // per domain (FP16 tiles), else null
+  const float* vfac;       // per vertex of block-diagonal domains
+  const float* bjinv;      // block Jacobi: 9 per vertex
+  const float* b;
+};
+
+// Host side of a solve: instance k covers vertices [vert[k], vert[k + 1]) and domains
+// [dom[k], dom[k + 1]), of which [diag[k], dom[k + 1]) are block diagonal.
+struct RsRun {
+  int precond = MGUSO_PRECOND_SCHWARZ;
+  bool mixed = true, half = false;
+  int sms = 148;
+  uint32_t nv = 0, ninst = 1;
+  uint64_t nnz = 0;  // blocks of A
+  uint32_t vert[PCG_MAX_INST + 1] = {}, dom[PCG_MAX_INST + 1] = {}, diag[PCG_MAX_INST] = {};
+};
+
+struct RsWork {
+  void* fn = nullptr;  // the kernel variant `smem` was found for
+  uint32_t smem = 0;   // its dynamic shared memory; 0: it cannot be resident on this device
+  DevBuf<float4> rec;
+  DevBuf<float> jscr;
+  DevBuf<uint4> sums;
+  DevBuf<uint32_t> count;
+  uint32_t epoch = 0;  // epochs used so far
+};
+
+// Solves the instances of `active` into x (3 floats per vertex; the others get x = 0) and
+// their results into out[k] (device), enqueued on st without a host wait. Returns
+// MGUSO_ERR_UNSUPPORTED, having enqueued nothing, when the system's vectors do not fit in the
+// SMs' shared memory (beyond about 64 domains or 2 000 vertices per SM).
+int pcg_resident(const RsSystem& sys, RsWork& w, const RsRun& run, float* x, uint32_t active, float tol,
+                 uint32_t max_iter, FusedInst* out, cudaStream_t st);
+
+// Domain ranges per instance of a one-level Schwarz preconditioner whose domains are grouped by
+// instance; false when they are not.
+bool resident_domains(const mguso_schwarz& s, RsRun& run);
+
 // Device vectors, scalars and the cached CUDA graph of one PCG operator.
 struct PcgWork {
   uint32_t n = 0;
-  DevBuf<float> b, x, r, z, p, ap, p2;  // p2: second direction buffer (persistent PCG)
+  DevBuf<float> b, x, r, z, p, ap, p2;  // p2: second direction buffer (fused PCG)
   DevBuf<PcgScalars> sc;
   DevBuf<double> partials;
   PcgScalars* h_sc = nullptr;  // pinned
@@ -220,6 +271,11 @@ struct mguso_linear_solver {
   std::unique_ptr<mguso_schwarz> schwarz;
   mg::DevBuf<float> bjinv;  // 9 per vertex (block Jacobi)
   mg::PcgWork work;
+  mg::RsWork rs;
+  mg::RsRun rs_run;
+  bool rs_ready = false;  // rs_run describes the cached pattern
+  mg::DevBuf<mg::FusedInst> rs_inst;
+  mg::PinnedBuf<mg::FusedInst> rs_out;
   uint64_t generation = 0;         // bumped whenever the pattern is rebuilt
   std::vector<uint32_t> map_val;   // scalar CSR entry -> BSR value slot
   std::vector<float> h_val;

@@ -227,10 +227,66 @@ int pcg_run(const PcgOps& ops, PcgWork& w, float tol, uint32_t max_iter, mguso_l
   return MGUSO_OK;
 }
 
+// The LinearSolver entry point's one-level system as one resident launch; UNSUPPORTED when it
+// is too large for it.
+static int pcg_solve_resident(mguso_linear_solver* s, float tol, uint32_t max_iter, mguso_lin_stats* out) {
+  mguso_bsr* a = s->bsr.get();
+  mguso_schwarz* sw = s->precond == MGUSO_PRECOND_SCHWARZ ? s->schwarz.get() : nullptr;
+  cudaStream_t st = s->ctx->stream;
+  RsRun& r = s->rs_run;
+  if (!s->rs_ready) {
+    r = RsRun{};
+    r.precond = s->precond;
+    r.mixed = s->precision == MGUSO_PRECISION_MIXED;
+    r.half = sw && sw->half;
+    r.sms = s->ctx->sm_count;
+    r.nv = a->nb;
+    r.nnz = a->nnzb;
+    r.vert[1] = a->nb;
+    if (sw && !resident_domains(*sw, r)) return MGUSO_ERR_UNSUPPORTED;
+    s->rs_ready = true;
+  }
+  RsSystem y{};
+  y.rp = a->row_ptr.p;
+  y.col = a->col.p;
+  y.val = a->val.p;
+  y.bjinv = s->bjinv.p;
+  y.b = s->work.b.p;
+  if (sw) {
+    y.dom_start = sw->dom_start.p;
+    y.dom_verts = sw->dom_verts.p;
+    y.vpos = sw->vpos.p;
+    y.fac_off = sw->fac_off.p;
+    y.fac = sw->half ? (const void*)sw->fac_h.p : (const void*)sw->fac.p;
+    y.fac_scale = sw->half ? sw->fac_scale.p : nullptr;
+    y.vfac = sw->vfac.p;
+  }
+  MG_TRY(s->rs_inst.reserve(1));
+  MG_TRY(s->rs_out.reserve(1));
+  MG_TRY(pcg_resident(y, s->rs, r, s->work.x.p, 1, tol, max_iter, s->rs_inst.p, st));
+  MG_CUDA(cudaMemcpyAsync(s->rs_out.p, s->rs_inst.p, sizeof(FusedInst), cudaMemcpyDeviceToHost, st));
+  MG_CUDA(cudaStreamSynchronize(st));
+  const FusedInst& o = *s->rs_out.p;
+  if (o.status & ST_WAIT_TIMEOUT) {
+    set_error("linear solve: a bounded wait between thread blocks timed out");
+    return MGUSO_ERR_TIMEOUT;
+  }
+  if (out) {
+    out->iters = o.iters;
+    out->residual = o.residual;
+    out->status = (o.residual <= tol || (o.status & ST_PCG_BREAKDOWN)) ? MGUSO_OK : MGUSO_ERR_PCG_CAP;
+  }
+  return MGUSO_OK;
+}
+
 // The LinearSolver entry point's system: the solver's own BSR and preconditioner.
 int pcg_solve(mguso_linear_solver* s, float tol, uint32_t max_iter, mguso_lin_stats* out) {
   mguso_bsr* a = s->bsr.get();
   MG_TRY(s->work.reserve(3 * a->nb));
+  if (s->levels != 2 && max_iter > 0 && a->nb > 0) {
+    const int rc = pcg_solve_resident(s, tol, max_iter, out);
+    if (rc != MGUSO_ERR_UNSUPPORTED) return rc;
+  }
   PcgOps ops;
   ops.stream = s->ctx->stream;
   ops.mixed = s->precision == MGUSO_PRECISION_MIXED;

@@ -1385,6 +1385,7 @@ extern "C" int mguso_scene_profile_pcg(mguso_scene* sc, int iters, float* us2, d
   } else {
     bytes2[1] = 36.0 * nv + 84.0 * nv;
   }
+  if (!s.schwarz || s.schwarz->levels != 2) MG_TRY(pcg_fused_select(s));
   return pcg_fused_profile(s, (uint32_t)iters, us2);
 }
 

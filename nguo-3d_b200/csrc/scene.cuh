@@ -177,14 +177,10 @@ struct Scene {
   DevBuf<unsigned long long> side_best;     // per vertex (d2 bits << 32 | tri)
   DevBuf<Stencil> stencils, stencils_sorted;
   uint32_t last_nst = 0;  // stencils of the last mguso_scene_assemble
-  // persistent PCG: grid (-1 until configured, 0 when it cannot be resident), barrier words,
-  // per-instance results and the instance row offsets
-  int pp_grid = -1;
-  DevBuf<uint32_t> pp_bar, pp_inst;
-  DevBuf<PcgInstResult> pp_out;
-  DevBuf<uint64_t> pp_probe;
-  DevBuf<double> pp_part;
-  std::vector<uint32_t> pp_key;  // instance rows the uploaded layout was built for
+  // resident PCG (pcg_resident.cu): scratch, and the instances' vertex and domain ranges
+  RsWork rs;
+  RsRun rs_run;
+  bool rs_ready = false;
   // fused two-kernel PCG: layout, per-instance state, partials and the cached graph
   std::vector<uint32_t> fr_key;
   std::vector<unsigned char> fr_graph_key;
@@ -266,7 +262,9 @@ int system_spmv(Scene& s, const float* p, float* ap, cudaStream_t st, const DotS
 // The instances' triangle and edge LBVHs at x; refit = true keeps each tree's shape from its
 // last build (the Newton iterations after a step's first) and only recomputes its boxes at x.
 int build_bvhs(Scene& s, const float* x, bool refit = false);
-int pcg_persistent(Scene& s, const uint32_t* h_inst_row, uint32_t ninst, uint32_t active, PcgInstResult* out);
+// The solve as one resident launch; its results are read with pcg_fused_results once the stream
+// has passed it. MGUSO_ERR_UNSUPPORTED (nothing enqueued) when the system is too large for it.
+int pcg_resident_scene(Scene& s, uint32_t active);
 // out == null defers the results: the caller synchronises the stream later and reads them with
 // pcg_fused_results (the solve itself never waits on the host)
 int pcg_fused(Scene& s, const uint32_t* h_inst_row, uint32_t ninst, uint32_t active, PcgInstResult* out);

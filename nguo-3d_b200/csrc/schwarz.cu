@@ -124,6 +124,9 @@ int schwarz_build(mguso_schwarz* s) {
   MG_TRY(s->dom_verts.upload(s->h_dom_verts.data(), s->h_dom_verts.size(), st));
   MG_TRY(s->dom_of.upload(s->h_dom_of.data(), nb, st));
   MG_TRY(s->loc.upload(loc.data(), nb, st));
+  std::vector<uint32_t> vpos(nb, 0);
+  for (uint32_t i = 0; i < (uint32_t)s->h_dom_verts.size(); ++i) vpos[s->h_dom_verts[i]] = i;
+  MG_TRY(s->vpos.upload(vpos.data(), nb, st));
   MG_TRY(s->fac_off.upload(off.data(), off.size(), st));
   if (s->half) {
     MG_TRY(s->fac_h.reserve(std::max<uint64_t>(s->fac_floats, 8)));

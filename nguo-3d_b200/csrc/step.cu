@@ -145,23 +145,23 @@ static int linear_solve(Scene& s, uint32_t active, mguso_lin_stats* ls, bool* de
   }
   const bool two_level = s.schwarz && s.schwarz->levels == 2;
   if (!two_level && (s.p.pcg_mode == 0 || s.p.pcg_mode == 2 || s.ninst > 1)) {
-    PcgInstResult r[PCG_MAX_INST] = {};
-    if (s.p.pcg_mode != 2) MG_TRY(pcg_fused_select(s));
-    const bool defer = deferred && s.p.pcg_mode != 2;
-    int rc = s.p.pcg_mode == 2 ? pcg_persistent(s, s.inst_vert.data(), s.ninst, active, r)
-                               : pcg_fused(s, s.inst_vert.data(), s.ninst, active, defer ? nullptr : r);
-    if (rc == MGUSO_OK) {
-      if (defer)
-        *deferred = true;
-      else
-        fused_stats(s, r, ls);
-      return MGUSO_OK;
+    // the resident kernel, unless the caller fixes a pair of fused kernels or the system is too
+    // large for it (batch step of six garments 157 ms against 214 ms with the fused kernels, one
+    // garment 39 against 74 ms for two steps, a 64 x 64 sheet 17 against 25 ms)
+    int rc = s.p.pcg_variant > 0 ? MGUSO_ERR_UNSUPPORTED : pcg_resident_scene(s, active);
+    if (rc == MGUSO_ERR_UNSUPPORTED) {
+      MG_TRY(pcg_fused_select(s));
+      rc = pcg_fused(s, s.inst_vert.data(), s.ninst, active, nullptr);
     }
-    if (rc != MGUSO_ERR_UNSUPPORTED) return rc;
-    if (s.ninst > 1) {
-      set_error("batched step: the persistent PCG cannot run on this device");
-      return MGUSO_ERR_UNSUPPORTED;
+    MG_TRY(rc);
+    if (deferred) {
+      *deferred = true;
+    } else {
+      PcgInstResult r[PCG_MAX_INST] = {};
+      MG_TRY(pcg_fused_results(s, s.ninst, r));
+      fused_stats(s, r, ls);
     }
+    return MGUSO_OK;
   }
   PcgOps ops;
   ops.stream = st;

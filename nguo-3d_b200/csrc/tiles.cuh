@@ -1,4 +1,4 @@
-// Schwarz factor storage shared by the standalone apply and the persistent PCG.
+// Schwarz factor storage shared by the standalone apply and the PCG kernels.
 #pragma once
 #include "internal.cuh"
 
