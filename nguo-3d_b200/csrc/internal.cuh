@@ -78,7 +78,6 @@ struct mguso_schwarz {
   mg::DevBuf<uint32_t> dom_start;  // ndom + 1 (vertex offsets)
   mg::DevBuf<uint32_t> dom_verts;  // nb
   mg::DevBuf<uint32_t> dom_of;     // nb
-  mg::DevBuf<uint32_t> loc;        // nb: local index of a vertex inside its domain
   mg::DevBuf<uint32_t> vpos;       // nb: a vertex's place in dom_verts
   mg::DevBuf<uint64_t> fac_off;    // ndom + 1 (float offsets, 4-float aligned)
   mg::DevBuf<float> fac;           // W = L^-1 per domain, swizzled 32x32 FP32 tiles
