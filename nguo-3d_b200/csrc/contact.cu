@@ -59,14 +59,6 @@ static BvhSet view_set(const std::vector<std::unique_ptr<Lbvh>>& b, const std::v
   return s;
 }
 
-template <class F>
-__device__ __forceinline__ bool visit(const BvhSet& bs, uint32_t k, float4 lo, float4 hi, F&& f) {
-  const BvhView& bv = bs.t[k];
-  const uint32_t base = bs.base[k];
-  return lbvh_visit(bv.left, bv.right, bv.node, bv.leaf, bv.prim, bv.n, lo, hi,
-                    [&](uint32_t local) { f(base + local); });
-}
-
 __device__ __forceinline__ void point_box(const float* x, uint32_t v, float pad, float4& lo, float4& hi) {
   float a = x[3 * v], b = x[3 * v + 1], c = x[3 * v + 2];
   lo = make_float4(__fsub_rn(a, pad), __fsub_rn(b, pad), __fsub_rn(c, pad), 0.f);
@@ -135,6 +127,157 @@ int build_bvhs(Scene& s, const float* x, bool refit) {
   return rc;
 }
 
+// ---- warp walks -------------------------------------------------------------------------------
+// A warp takes `per` consecutive queries (up to 32) down their trees together: its queue holds
+// (query, node) pairs, each round takes up to 32 of them, newest first, one per lane, tests the
+// node's two children against the query and queues those entered; leaves go, as (query,
+// primitive) pairs, to a second queue, from which the whole warp takes 32 at a time through the
+// remaining filters and the narrow phase (distances, accd_toi). What bounds a walk is its chain
+// of dependent rounds: with a stack per lane, a warp ran as many rounds as its longest query
+// has nodes (some hundreds, about half of the lanes idle), while a shared queue keeps all
+// lanes on nodes of any query and needs little more than their number over 32, so that few
+// queries per warp (small scenes) spread over more warps. 64 x 64 sheet, before -> after: edge-edge
+// CCD 219 -> 87 us, vertex-triangle CCD 150 -> 30, stencils 140 -> 40 and 97 -> 22; one garment:
+// 160 -> 129, 176 -> 98, 145 -> 94 and 140 -> 49; six garments: 522 -> 421, 320 -> 243,
+// 408 -> 302 and 205 -> 122.
+// Results are order-free: stencils are sorted by their pair key afterwards, CCD results are
+// minima and sums, and the leaves reached do not depend on the order of the tests.
+constexpr int WQ_WARPS = 4;   // 128-thread blocks
+constexpr int WQ_QCAP = 96;   // < 32 left over + 2 leaves per lane and round
+// queued nodes per warp: a round adds at most 32; past FW_FULL one node is taken at a time, which
+// goes down depth first and adds at most one per level
+constexpr int FW_CAP = 1024, FW_FULL = FW_CAP - 128;
+
+template <class Q>
+struct WalkMem {  // shared memory of one warp
+  Q query[32];
+  uint32_t node[FW_CAP];
+  uint2 pair[WQ_QCAP];
+  uint8_t slot[FW_CAP];
+  uint8_t inst[32];
+};
+
+__device__ __forceinline__ void wq_push(uint2* q, int& n, bool has, uint2 e) {
+  const unsigned m = __ballot_sync(0xffffffffu, has);
+  if (has) q[n + __popc(m & ((1u << (threadIdx.x & 31)) - 1u))] = e;
+  n += __popc(m);
+}
+
+// Takes batches of up to 32 queued pairs while at least min_n are queued (n is warp-uniform).
+template <class F>
+__device__ __forceinline__ void wq_take(uint2* q, int& n, int min_n, F&& solve) {
+  const int lane = (int)(threadIdx.x & 31);
+  __syncwarp();
+  while (n >= min_n && n > 0) {
+    const int take = n < 32 ? n : 32;
+    const bool has = lane < take;
+    const uint2 e = has ? q[n - take + lane] : make_uint2(0u, 0u);
+    __syncwarp();
+    n -= take;
+    if (has) solve(e);
+  }
+}
+
+// Walks the trees of the warp's queries: lane l holds query l (valid or not) of instance k,
+// numbered first + l. keep(slot, primitive) says whether a leaf reached is to be solved.
+// Returns false when the node queue overflowed.
+template <class Q, class KEEP, class SOLVE>
+__device__ __forceinline__ bool warp_walk(WalkMem<Q>& m, const BvhSet& bs, uint32_t first, bool valid, uint32_t k,
+                                          const Q& mine, KEEP&& keep, SOLVE&& solve) {
+  const int lane = (int)(threadIdx.x & 31);
+  const unsigned below = (1u << lane) - 1u;
+  int n = 0, np = 0;
+  bool ok = true;
+  if (valid) {
+    m.query[lane] = mine;
+    m.inst[lane] = (uint8_t)k;
+  }
+  __syncwarp();
+  {
+    bool root = false, leaf = false;
+    uint32_t prim = 0;
+    if (valid) {
+      const BvhView& t = bs.t[k];
+      if (t.n == 1) {
+        leaf = mine.enter(__ldg(t.leaf), __ldg(t.leaf + 1), t.dleaf);
+        prim = bs.base[k] + __ldg(t.prim);
+      } else if (t.n > 1) {
+        root = mine.enter(__ldg(t.node), __ldg(t.node + 1), t.dnode);
+      }
+    }
+    const unsigned r = __ballot_sync(0xffffffffu, root);
+    if (root) {
+      const int at = __popc(r & below);
+      m.node[at] = 0;
+      m.slot[at] = (uint8_t)lane;
+    }
+    n = __popc(r);
+    if (leaf) leaf = keep((uint32_t)lane, prim);
+    wq_push(m.pair, np, leaf, make_uint2(first + lane, prim));
+  }
+  __syncwarp();
+  while (n > 0) {
+    const int take = n <= FW_FULL ? min(n, 32) : 1;
+    if (n + take > FW_CAP) {
+      ok = false;
+      break;
+    }
+    const bool has = lane < take;
+    uint32_t ch[2] = {0, 0}, slot = 0, base = 0;
+    const uint32_t* prims = nullptr;
+    bool in[2] = {false, false};
+    if (has) {
+      const uint32_t cur = m.node[n - take + lane];
+      slot = m.slot[n - take + lane];
+      const BvhView& t = bs.t[m.inst[slot]];
+      base = bs.base[m.inst[slot]];
+      prims = t.prim;
+      ch[0] = __ldg(t.left + cur);
+      ch[1] = __ldg(t.right + cur);
+      const float4* cb = t.cbox + 4 * (size_t)cur;
+      const float4* db = t.dcbox + 4 * (size_t)cur;
+      const float4 l0 = __ldg(cb), h0 = __ldg(cb + 1), l1 = __ldg(cb + 2), h1 = __ldg(cb + 3);
+      const Q& q = m.query[slot];
+      in[0] = q.enter(l0, h0, db);
+      in[1] = q.enter(l1, h1, db + 2);
+    }
+    n -= take;
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const bool inner = in[c] && !(ch[c] & LEAF_BIT);
+      const unsigned b = __ballot_sync(0xffffffffu, inner);
+      if (inner) {
+        const int at = n + __popc(b & below);
+        m.node[at] = ch[c];
+        m.slot[at] = (uint8_t)slot;
+      }
+      n += __popc(b);
+      bool leaf = in[c] && (ch[c] & LEAF_BIT);
+      uint32_t prim = 0;
+      if (leaf) {
+        prim = base + __ldg(prims + (ch[c] & ~LEAF_BIT));
+        leaf = keep(slot, prim);
+      }
+      wq_push(m.pair, np, leaf, make_uint2(first + slot, prim));
+    }
+    wq_take(m.pair, np, 32, solve);
+    __syncwarp();
+  }
+  wq_take(m.pair, np, 1, solve);
+  return ok;
+}
+
+// Queries per warp: as many as leave every SM some warps (a walk's rounds are latency-bound), up
+// to the 32 that fill a round from its start.
+static uint32_t walk_per(const Scene& s, uint32_t n) {
+  const uint64_t fill = 16ull * (uint64_t)s.ctx->sm_count;
+  uint32_t per = 32;
+  while (per > 4 && (uint64_t)n < fill * per) per /= 2;
+  return per;
+}
+static uint32_t walk_grid(uint32_t n, uint32_t per) { return ceil_div(n, WQ_WARPS * per); }
+
 // ---- self intersection (has_self_intersection, implicit.rs:618-650) ------------------
 // edge_triangle_intersect (contact.rs:324-352) in FP32, in the reference's operation order
 // (this file is compiled without FMA contraction): the segment crosses the triangle's plane
@@ -158,26 +301,31 @@ __device__ __forceinline__ bool edge_triangle_intersect_f(V3<float> e0, V3<float
 // Every mesh edge against the triangles whose boxes overlap its own box (every piercing
 // pair is among them): pairs with a movable vertex that share no vertex, counted per
 // instance into red[RED_STRIDE k + 14].
-__global__ void k_self_intersect(BvhSet bv, const uint8_t* __restrict__ vinst, const float* __restrict__ x,
-                                 const uint32_t* __restrict__ edges, const uint32_t* __restrict__ tris,
-                                 const float* __restrict__ im, uint32_t ne, unsigned int* __restrict__ red,
-                                 uint32_t* status) {
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= ne) return;
-  const uint32_t e0 = edges[2 * j], e1 = edges[2 * j + 1];
-  float4 lo, hi;
-  edge_box(x, e0, e1, 0.f, lo, hi);
-  const bool emov = im[e0] > 0.f || im[e1] > 0.f;
-  const V3<float> p0 = ld3<float>(x, e0), p1 = ld3<float>(x, e1);
-  unsigned int hits = 0;
-  const bool ok = visit(bv, vinst[e0], lo, hi, [&](uint32_t t) {
-    const uint32_t a = tris[3 * t], b = tris[3 * t + 1], c = tris[3 * t + 2];
-    if (!emov && !(im[a] > 0.f || im[b] > 0.f || im[c] > 0.f)) return;
+__global__ void __launch_bounds__(WQ_WARPS * 32) k_self_intersect(
+    BvhSet bv, const uint8_t* __restrict__ vinst, const float* __restrict__ x, const uint32_t* __restrict__ edges,
+    const uint32_t* __restrict__ tris, const float* __restrict__ im, uint32_t ne, uint32_t per,
+    unsigned int* __restrict__ red, uint32_t* status) {
+  __shared__ WalkMem<BoxQuery> mem[WQ_WARPS];
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, first = (blockIdx.x * WQ_WARPS + w) * per;
+  const uint32_t j = first + lane;
+  const bool valid = lane < per && j < ne;
+  BoxQuery q;
+  uint32_t k = 0;
+  if (valid) {
+    const uint32_t e0 = edges[2 * j], e1 = edges[2 * j + 1];
+    k = vinst[e0];
+    edge_box(x, e0, e1, 0.f, q.lo, q.hi);
+  }
+  const bool ok = warp_walk(mem[w], bv, first, valid, k, q, [](uint32_t, uint32_t) { return true; }, [&](uint2 e) {
+    const uint32_t e0 = edges[2 * e.x], e1 = edges[2 * e.x + 1];
+    const uint32_t a = tris[3 * e.y], b = tris[3 * e.y + 1], c = tris[3 * e.y + 2];
+    if (!(im[e0] > 0.f || im[e1] > 0.f || im[a] > 0.f || im[b] > 0.f || im[c] > 0.f)) return;
     if (e0 == a || e0 == b || e0 == c || e1 == a || e1 == b || e1 == c) return;
-    if (edge_triangle_intersect_f(p0, p1, ld3<float>(x, a), ld3<float>(x, b), ld3<float>(x, c))) ++hits;
+    if (edge_triangle_intersect_f(ld3<float>(x, e0), ld3<float>(x, e1), ld3<float>(x, a), ld3<float>(x, b),
+                                  ld3<float>(x, c)))
+      atomicAdd(red + RED_STRIDE * vinst[e0] + 14, 1u);
   });
   if (!ok) atomicOr(status, ST_STACK_OVERFLOW);
-  if (hits) atomicAdd(red + RED_STRIDE * vinst[e0] + 14, hits);
 }
 
 // Piercing (edge, triangle) pairs of every instance at the scene's positions x, counted into
@@ -196,8 +344,9 @@ int self_intersections(Scene& s, bool refit) {
   MG_TRY(aux_join(s));
   MG_TRY(rc);
   BvhSet tv = view_set(s.tri_bvh, s.inst_tri);
-  k_self_intersect<<<ceil_div(s.n_edge, 128), 128, 0, s.st>>>(tv, s.vinst.p, s.x.p, s.edges.p, s.tris.p, s.inv_mass.p,
-                                                             s.n_edge, s.red.p, s.status.p);
+  const uint32_t per = walk_per(s, s.n_edge);
+  k_self_intersect<<<walk_grid(s.n_edge, per), WQ_WARPS * 32, 0, s.st>>>(
+      tv, s.vinst.p, s.x.p, s.edges.p, s.tris.p, s.inv_mass.p, s.n_edge, per, s.red.p, s.status.p);
   MG_CUDA(cudaGetLastError());
   return MGUSO_OK;
 }
@@ -206,31 +355,38 @@ int self_intersections(Scene& s, bool refit) {
 // best (d2 bits, triangle) per non-static vertex over collider triangles within dhat; ties
 // go to the lowest triangle index, which is the first one the reference's triangle-major
 // visit reaches.
-__global__ void k_side_best(BvhSet bv, const uint8_t* __restrict__ vinst, const float* __restrict__ x, const uint32_t* __restrict__ tris,
-                            const uint8_t* __restrict__ ctri, const uint8_t* __restrict__ svert,
-                            const float* __restrict__ im, const uint32_t* __restrict__ ex_ptr,
-                            const uint32_t* __restrict__ ex_list, uint32_t nv, float dhat,
-                            unsigned long long* __restrict__ best, uint32_t* __restrict__ status, uint32_t active) {
-  uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= nv || !((active >> vinst[v]) & 1u)) return;
-  unsigned long long b = ~0ull;
-  if (!svert[v] && im[v] > 0.f) {
-    float4 lo, hi;
-    point_box(x, v, dhat, lo, hi);
-    V3<float> p = ld3<float>(x, v);
-    bool ok = visit(bv, vinst[v], lo, hi, [&](uint32_t t) {
-      if (!ctri[t]) return;
-      uint32_t a = tris[3 * t], bb = tris[3 * t + 1], c = tris[3 * t + 2];
-      if (excluded(ex_ptr, ex_list, v, a, bb, c)) return;
-      float w[3];
-      V3<float> q = closest_point_bary(p, ld3<float>(x, a), ld3<float>(x, bb), ld3<float>(x, c), w);
-      float d2 = (p - q).length_squared();
-      unsigned long long k = ((unsigned long long)__float_as_uint(d2) << 32) | t;
-      if (k < b) b = k;
-    });
-    if (!ok) atomicOr(status, ST_STACK_OVERFLOW);
+__global__ void __launch_bounds__(WQ_WARPS * 32) k_side_best(
+    BvhSet bv, const uint8_t* __restrict__ vinst, const float* __restrict__ x, const uint32_t* __restrict__ tris,
+    const uint8_t* __restrict__ ctri, const uint8_t* __restrict__ svert, const float* __restrict__ im,
+    const uint32_t* __restrict__ ex_ptr, const uint32_t* __restrict__ ex_list, uint32_t nv, float dhat, uint32_t per,
+    unsigned long long* __restrict__ best, uint32_t* __restrict__ status, uint32_t active) {
+  __shared__ WalkMem<BoxQuery> mem[WQ_WARPS];
+  __shared__ unsigned long long s_best[WQ_WARPS][32];
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, first = (blockIdx.x * WQ_WARPS + w) * per;
+  const uint32_t v = first + lane;
+  const bool mine = lane < per && v < nv && ((active >> vinst[v]) & 1u);
+  const bool valid = mine && !svert[v] && im[v] > 0.f;
+  BoxQuery q;
+  uint32_t k = 0;
+  if (valid) {
+    k = vinst[v];
+    point_box(x, v, dhat, q.lo, q.hi);
   }
-  best[v] = b;
+  s_best[w][lane] = ~0ull;
+  const bool ok = warp_walk(mem[w], bv, first, valid, k, q, [&](uint32_t, uint32_t t) { return ctri[t] != 0; },
+                            [&](uint2 e) {
+    const uint32_t qv = e.x, t = e.y;
+    const uint32_t a = tris[3 * t], b = tris[3 * t + 1], c = tris[3 * t + 2];
+    if (excluded(ex_ptr, ex_list, qv, a, b, c)) return;
+    float bary[3];
+    const V3<float> p = ld3<float>(x, qv);
+    const V3<float> cp = closest_point_bary(p, ld3<float>(x, a), ld3<float>(x, b), ld3<float>(x, c), bary);
+    const float d2 = (p - cp).length_squared();
+    atomicMin(&s_best[w][qv - first], ((unsigned long long)__float_as_uint(d2) << 32) | t);
+  });
+  __syncwarp();
+  if (!ok) atomicOr(status, ST_STACK_OVERFLOW);
+  if (mine) best[v] = s_best[w][lane];
 }
 
 __device__ __forceinline__ float side_of(uint32_t v, const unsigned long long* best, const float* x,
@@ -271,38 +427,6 @@ __device__ __forceinline__ void emit_stencil(Stencil* out, unsigned long long* k
   ids[at] = (uint32_t)at;
 }
 
-// ---- warp-pooled narrow phase ---------------------------------------------------------------
-// Each lane walks its query's tree (BoxWalk, CcdWalk) and pushes the leaves it reaches, as
-// (query, primitive) pairs, onto its warp's queue in shared memory; whenever 32 are queued the
-// whole warp takes them, one per lane, through the remaining filters and the narrow phase
-// (distances, accd_toi). The walks stay per lane, but the narrow phase (the bulk of the work)
-// runs on full warps instead of on the few lanes whose walk happens to sit on a leaf. Its
-// results are order-free: stencils are sorted by their pair key afterwards, CCD results are
-// per (instance, pass) minima and sums.
-constexpr int WQ_WARPS = 4;   // 128-thread blocks
-constexpr int WQ_QCAP = 96;   // < 32 left over + 2 leaves per lane and step
-
-__device__ __forceinline__ void wq_push(uint2* q, int& n, bool has, uint2 e) {
-  const unsigned m = __ballot_sync(0xffffffffu, has);
-  if (has) q[n + __popc(m & ((1u << (threadIdx.x & 31)) - 1u))] = e;
-  n += __popc(m);
-}
-
-// Takes batches of up to 32 queued pairs while at least min_n are queued (n is warp-uniform).
-template <class F>
-__device__ __forceinline__ void wq_take(uint2* q, int& n, int min_n, F&& solve) {
-  const int lane = (int)(threadIdx.x & 31);
-  __syncwarp();
-  while (n >= min_n && n > 0) {
-    const int take = n < 32 ? n : 32;
-    const bool has = lane < take;
-    const uint2 e = has ? q[n - take + lane] : make_uint2(0u, 0u);
-    __syncwarp();
-    n -= take;
-    if (has) solve(e);
-  }
-}
-
 template <class R>
 __device__ __forceinline__ R vt_distance(const float* x, const uint32_t idx[4], bool collider, bool inside, R g[12]) {
   V3<R> gg[4];
@@ -323,40 +447,24 @@ __device__ __forceinline__ R ee_distance(const float* x, const uint32_t idx[4], 
   return d;
 }
 
-// Vertex-triangle pairs: lane v walks the triangles near vertex v; the distances run pooled
-// per warp. A static collider triangle needs v's side of the collider, which depends on v
-// alone (side_of), so the lane that takes the pair evaluates it.
+// Vertex-triangle pairs: query v is vertex v. A static collider triangle needs v's side of the
+// collider, which depends on v alone (side_of), so the lane that takes the pair evaluates it.
 __global__ void __launch_bounds__(WQ_WARPS * 32) k_vt_stencils(
     BvhSet bv, const uint8_t* __restrict__ vinst, const float* __restrict__ x, const uint32_t* __restrict__ tris,
     const uint8_t* __restrict__ ctri, const float* __restrict__ im, const uint32_t* __restrict__ ex_ptr,
     const uint32_t* __restrict__ ex_list, const unsigned long long* __restrict__ best, const float* __restrict__ pn,
     int has_static, uint32_t nv, float dhat, int mixed, Stencil* out, unsigned long long* keys, uint32_t* ids,
-    unsigned long long* counter, uint32_t cap, uint32_t* status, uint32_t active) {
-  __shared__ uint2 qbuf[WQ_WARPS][WQ_QCAP];
-  uint2* q = qbuf[threadIdx.x >> 5];
-  int qn = 0;
-  const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t base = 0;
-  bool done = true;
-  BoxWalk walk;
-  walk.ok = true;
-  uint32_t outp[2];
-  int nout = 0;
-  if (v < nv) {
-    const uint32_t k = vinst[v];
-    if ((active >> k) & 1u) {
-      const BvhView& tv = bv.t[k];
-      base = bv.base[k];
-      walk.left = tv.left;
-      walk.right = tv.right;
-      walk.prim = tv.prim;
-      walk.node = tv.node;
-      walk.leaf = tv.leaf;
-      walk.cbox = tv.cbox;
-      walk.nt = tv.n;
-      point_box(x, v, dhat, walk.qlo, walk.qhi);
-      nout = walk.start(done, outp);
-    }
+    unsigned long long* counter, uint32_t cap, uint32_t* status, uint32_t active, uint32_t per) {
+  __shared__ WalkMem<BoxQuery> mem[WQ_WARPS];
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, first = (blockIdx.x * WQ_WARPS + w) * per;
+  const uint32_t v = first + lane;
+  BoxQuery q;
+  uint32_t k = 0;
+  bool valid = false;
+  if (lane < per && v < nv) {
+    k = vinst[v];
+    valid = ((active >> k) & 1u) != 0;
+    if (valid) point_box(x, v, dhat, q.lo, q.hi);
   }
   auto solve = [&](uint2 e) {
     const uint32_t qv = e.x, t = e.y;
@@ -375,55 +483,30 @@ __global__ void __launch_bounds__(WQ_WARPS * 32) k_vt_stencils(
     if (!(d < (double)dhat)) return;
     emit_stencil(out, keys, ids, counter, cap, status, 0, qv, t, idx, d, dhat, g);
   };
-  for (;;) {
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const bool leaf = c < nout;
-      wq_push(q, qn, leaf, make_uint2(v, leaf ? base + outp[c] : 0u));
-    }
-    wq_take(q, qn, 32, solve);
-    if (!__any_sync(0xffffffffu, !done)) break;
-    nout = done ? 0 : walk.step(done, outp);
-  }
-  wq_take(q, qn, 1, solve);
-  if (!walk.ok) atomicOr(status, ST_STACK_OVERFLOW);
+  if (!warp_walk(mem[w], bv, first, valid, k, q, [](uint32_t, uint32_t) { return true; }, solve))
+    atomicOr(status, ST_STACK_OVERFLOW);
 }
 
-// Edge-edge pairs: lane t (edge t) takes the pairs (t, p) with p > t, the lower-indexed edge
+// Edge-edge pairs: query t is edge t, for the pairs (t, p) with p > t, the lower-indexed edge
 // first in the stencil and its key, so each pair is seen once. An edge in its instance's static
 // tail (every edge from there on has both vertices pinned) has no partner above it that can
-// move, and skips its walk. The distances run pooled per warp.
+// move, and skips its walk.
 __global__ void __launch_bounds__(WQ_WARPS * 32) k_ee_stencils(
     BvhSet bv, const uint8_t* __restrict__ vinst, const float* __restrict__ x, const uint32_t* __restrict__ edges,
     const uint32_t* __restrict__ ee_tail, const float* __restrict__ im, uint32_t ne, float search, float dhat,
     int mixed, Stencil* out, unsigned long long* keys, uint32_t* ids, unsigned long long* counter, uint32_t cap,
-    uint32_t* status, uint32_t active) {
-  __shared__ uint2 qbuf[WQ_WARPS][WQ_QCAP];
-  uint2* q = qbuf[threadIdx.x >> 5];
-  int qn = 0;
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t base = 0;
-  bool done = true;
-  BoxWalk walk;
-  walk.ok = true;
-  uint32_t outp[2];
-  int nout = 0;
-  if (t < ne) {
+    uint32_t* status, uint32_t active, uint32_t per) {
+  __shared__ WalkMem<BoxQuery> mem[WQ_WARPS];
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, first = (blockIdx.x * WQ_WARPS + w) * per;
+  const uint32_t t = first + lane;
+  BoxQuery q;
+  uint32_t k = 0;
+  bool valid = false;
+  if (lane < per && t < ne) {
     const uint32_t b0 = edges[2 * t], b1 = edges[2 * t + 1];
-    const uint32_t k = vinst[b0];
-    if (t < ee_tail[k] && ((active >> k) & 1u)) {
-      const BvhView& tv = bv.t[k];
-      base = bv.base[k];
-      walk.left = tv.left;
-      walk.right = tv.right;
-      walk.prim = tv.prim;
-      walk.node = tv.node;
-      walk.leaf = tv.leaf;
-      walk.cbox = tv.cbox;
-      walk.nt = tv.n;
-      edge_box(x, b0, b1, search, walk.qlo, walk.qhi);
-      nout = walk.start(done, outp);
-    }
+    k = vinst[b0];
+    valid = t < ee_tail[k] && ((active >> k) & 1u);
+    if (valid) edge_box(x, b0, b1, search, q.lo, q.hi);
   }
   auto solve = [&](uint2 e) {
     const uint32_t qt = e.x, p = e.y;
@@ -441,19 +524,8 @@ __global__ void __launch_bounds__(WQ_WARPS * 32) k_ee_stencils(
     if (!(d < ghat)) return;
     emit_stencil(out, keys, ids, counter, cap, status, 1, qt, p, idx, d, ghat, g);
   };
-  for (;;) {
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const bool leaf = c < nout;
-      const uint32_t p = leaf ? base + outp[c] : 0u;
-      wq_push(q, qn, leaf && p > t, make_uint2(t, p));
-    }
-    wq_take(q, qn, 32, solve);
-    if (!__any_sync(0xffffffffu, !done)) break;
-    nout = done ? 0 : walk.step(done, outp);
-  }
-  wq_take(q, qn, 1, solve);
-  if (!walk.ok) atomicOr(status, ST_STACK_OVERFLOW);
+  if (!warp_walk(mem[w], bv, first, valid, k, q, [&](uint32_t slot, uint32_t p) { return p > first + slot; }, solve))
+    atomicOr(status, ST_STACK_OVERFLOW);
 }
 
 __global__ void k_permute_stencils(const Stencil* __restrict__ in, const uint32_t* __restrict__ ids, uint32_t n,
@@ -466,10 +538,11 @@ int collect_stencils(Scene& s, uint32_t* nst_out) {
   cudaStream_t st = s.st;
   const float dhat = s.p.contact_dhat;
   const BvhSet tv = view_set(s.tri_bvh, s.inst_tri), ev = view_set(s.edge_bvh, s.inst_edge);
+  const uint32_t vper = walk_per(s, s.nv), eper = walk_per(s, s.n_edge);
   if (s.has_static) {
-    k_side_best<<<ceil_div(s.nv, 128), 128, 0, st>>>(tv, s.vinst.p, s.x.p, s.tris.p, s.collider_tri.p, s.static_vert.p,
-                                                   s.inv_mass.p, s.ex_ptr.p, s.ex_list.p, s.nv, dhat, s.side_best.p,
-                                                   s.status.p, s.iter_active);
+    k_side_best<<<walk_grid(s.nv, vper), WQ_WARPS * 32, 0, st>>>(
+        tv, s.vinst.p, s.x.p, s.tris.p, s.collider_tri.p, s.static_vert.p, s.inv_mass.p, s.ex_ptr.p, s.ex_list.p, s.nv,
+        dhat, vper, s.side_best.p, s.status.p, s.iter_active);
   }
   for (int attempt = 0; attempt < 4; ++attempt) {
     MG_TRY(s.stencils.reserve(s.cap_stencils));
@@ -480,14 +553,14 @@ int collect_stencils(Scene& s, uint32_t* nst_out) {
     // the two kinds run concurrently on side streams (they share the output through its
     // atomic counter; the stencils are put in key order below)
     MG_TRY(aux_fork(s));
-    k_vt_stencils<<<ceil_div(s.nv, 128), 128, 0, s.aux[0]>>>(
+    k_vt_stencils<<<walk_grid(s.nv, vper), WQ_WARPS * 32, 0, s.aux[0]>>>(
         tv, s.vinst.p, s.x.p, s.tris.p, s.collider_tri.p, s.inv_mass.p, s.ex_ptr.p, s.ex_list.p, s.side_best.p,
         s.collider_pn.p, s.has_static ? 1 : 0, s.nv, dhat, s.mixed ? 1 : 0, s.stencils.p, s.st_keys.p, s.st_ids.p,
-        s.counters.p, s.cap_stencils, s.status.p, s.iter_active);
+        s.counters.p, s.cap_stencils, s.status.p, s.iter_active, vper);
     if (s.n_edge)
-      k_ee_stencils<<<ceil_div(s.n_edge, 128), 128, 0, s.aux[1]>>>(
+      k_ee_stencils<<<walk_grid(s.n_edge, eper), WQ_WARPS * 32, 0, s.aux[1]>>>(
           ev, s.vinst.p, s.x.p, s.edges.p, s.ee_tail.p, s.inv_mass.p, s.n_edge, dhat, dhat, s.mixed ? 1 : 0,
-          s.stencils.p, s.st_keys.p, s.st_ids.p, s.counters.p, s.cap_stencils, s.status.p, s.iter_active);
+          s.stencils.p, s.st_keys.p, s.st_ids.p, s.counters.p, s.cap_stencils, s.status.p, s.iter_active, eper);
     MG_CUDA(cudaGetLastError());
     MG_TRY(aux_join(s));
     unsigned long long cnt = 0;
@@ -624,7 +697,7 @@ __global__ void k_ccd_sl(uint32_t n, const uint32_t* __restrict__ fv, const floa
 
 // CCD candidate pruning: a pair whose accd_toi (contact.rs:378-437) would return max_t at
 // its first test cannot lower the step fraction, and traversal skips whole subtrees of such
-// pairs (CcdWalk) from the primitives' displacement boxes, refitted per CCD call.
+// pairs (CcdQuery) from the primitives' displacement boxes, refitted per CCD call.
 
 // Per-instance CCD passes of one launch: up to CCD_CHUNK consecutive search radii of the
 // widening schedule (ascending). The traversal uses the largest; each candidate pair's ACCD
@@ -710,59 +783,52 @@ struct CcdAcc {
   }
 };
 
-__device__ __forceinline__ void walk_init(CcdWalk& w, const BvhSet& bs, uint32_t k, float4 lo, float4 hi, float4 qlo,
-                                          float4 qhi, float3 cq, float rq) {
-  const BvhView& bv = bs.t[k];
-  w.left = bv.left;
-  w.right = bv.right;
-  w.prim = bv.prim;
-  w.node = bv.node;
-  w.leaf = bv.leaf;
-  w.dnode = bv.dnode;
-  w.dleaf = bv.dleaf;
-  w.cbox = bv.cbox;
-  w.dcbox = bv.dcbox;
-  w.nt = bv.n;
-  w.slo = lo;
-  w.shi = hi;
-  w.qlo = qlo;
-  w.qhi = qhi;
-  w.cq = cq;
-  w.rq = rq;
-}
+// Adds a walk's leaf count to its instance's diagnostics, instance by instance.
+struct LeafCount {
+  uint32_t k, n;
+  unsigned int* red;
+  int slot;
+  __device__ __forceinline__ void add(uint32_t kk) {
+    if (kk != k) {
+      flush();
+      k = kk;
+    }
+    ++n;
+  }
+  __device__ __forceinline__ void flush() {
+    if (n) atomicAdd(red + RED_STRIDE * k + slot, n);
+    n = 0;
+  }
+};
 
-// Vertex-triangle passes: lane v walks the triangles near vertex v.
+// Vertex-triangle passes: query v is vertex v.
 template <class R>
 __global__ void __launch_bounds__(WQ_WARPS * 32, 4) k_ccd_vt(
     BvhSet bv, const CcdPass* __restrict__ cpp, const uint8_t* __restrict__ vinst, const float* __restrict__ x,
     const float* __restrict__ dx, const uint32_t* __restrict__ tris, const uint8_t* __restrict__ ctri,
     const float* __restrict__ im, const uint32_t* __restrict__ ex_ptr, const uint32_t* __restrict__ ex_list,
     const unsigned long long* __restrict__ best, const float* __restrict__ pn, int has_static, uint32_t nv, float dhat,
-    uint32_t max_iter, unsigned int* __restrict__ red, unsigned int* __restrict__ acc, uint32_t* __restrict__ status) {
-  __shared__ uint2 qbuf[WQ_WARPS][WQ_QCAP];
-  uint2* q = qbuf[threadIdx.x >> 5];
-  int qn = 0;
+    uint32_t max_iter, unsigned int* __restrict__ red, unsigned int* __restrict__ acc, uint32_t* __restrict__ status,
+    uint32_t per) {
+  __shared__ WalkMem<CcdQuery> mem[WQ_WARPS];
+  __shared__ float s_side[WQ_WARPS][32];  // of the collider, per vertex (2: not yet known)
   const CcdPass& cp = *cpp;
-  const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t k = 0xffffffffu, base = 0, nleaf = 0;
-  bool done = true;
-  float side = 2.f;
-  CcdWalk walk;
-  walk.ok = true;
-  uint32_t out[2];
-  int nout = 0;
-  if (v < nv) {
-    const uint32_t kv = vinst[v];
-    if ((cp.todo >> kv) & 1u) {
-      k = kv;
-      base = bv.base[k];
-      float4 lo, hi, qlo, qhi;
-      point_box(x, v, cp.search[k][cp.npass[k] - 1], lo, hi);
-      point_box(x, v, 0.f, qlo, qhi);
-      walk_init(walk, bv, k, lo, hi, qlo, qhi, make_float3(dx[3 * v], dx[3 * v + 1], dx[3 * v + 2]), 0.f);
-      nout = walk.start(done, out);
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, first = (blockIdx.x * WQ_WARPS + w) * per;
+  const uint32_t v = first + lane;
+  CcdQuery q;
+  uint32_t k = 0;
+  bool valid = false;
+  s_side[w][lane] = 2.f;
+  if (lane < per && v < nv) {
+    k = vinst[v];
+    valid = ((cp.todo >> k) & 1u) != 0;
+    if (valid) {
+      point_box(x, v, cp.search[k][cp.npass[k] - 1], q.slo, q.shi);
+      point_box(x, v, 0.f, q.qlo, q.qhi);
+      q.c = make_float4(dx[3 * v], dx[3 * v + 1], dx[3 * v + 2], 0.f);
     }
   }
+  LeafCount nleaf{0u, 0u, red, 5};
   CcdAcc a;
   a.reset(0xffffffffu);
   auto solve = [&](uint2 e) {
@@ -788,69 +854,55 @@ __global__ void __launch_bounds__(WQ_WARPS * 32, 4) k_ccd_vt(
     const R toi = accd_toi<R>(x0, dd, R(0), R(1.25), R(0.01), max_iter, 0, &capped);
     a.add(kq, i0, (float)(toi / R(1.25)), capped, cp, acc, red, 6);
   };
-  for (;;) {
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      bool has = c < nout;
-      const uint32_t t = has ? base + out[c] : 0u;
-      if (has) {
-        ++nleaf;
-        // a collider triangle only counts on the vertex's outer side (lazily, once per vertex)
-        if (has_static && ctri[t]) {
-          if (side == 2.f) side = side_of(v, best, x, tris, pn, dhat);
-          if (side < 0.f) has = false;
-        }
+  auto keep = [&](uint32_t slot, uint32_t t) {
+    nleaf.add(mem[w].inst[slot]);
+    // a collider triangle only counts on the vertex's outer side (found once per vertex)
+    if (has_static && ctri[t]) {
+      float side = s_side[w][slot];
+      if (side == 2.f) {
+        side = side_of(first + slot, best, x, tris, pn, dhat);
+        s_side[w][slot] = side;
       }
-      wq_push(q, qn, has, make_uint2(v, t));
+      if (side < 0.f) return false;
     }
-    wq_take(q, qn, 32, solve);
-    if (!__any_sync(0xffffffffu, !done)) break;
-    nout = done ? 0 : walk.step(done, out);
-  }
-  wq_take(q, qn, 1, solve);
+    return true;
+  };
+  if (!warp_walk(mem[w], bv, first, valid, k, q, keep, solve)) atomicOr(status, ST_STACK_OVERFLOW);
   a.flush(cp, acc, red, 6);
-  if (!walk.ok) atomicOr(status, ST_STACK_OVERFLOW);
-  if (nleaf) atomicAdd(red + RED_STRIDE * k + 5, nleaf);
+  nleaf.flush();
 }
 
-// Edge-edge passes. As k_ee_stencils: lane j takes the pairs (j, i) with i > j (the
+// Edge-edge passes. As k_ee_stencils: query j takes the pairs (j, i) with i > j (the
 // lower-indexed edge first), and an edge of its instance's static tail skips its walk.
 template <class R>
 __global__ void __launch_bounds__(WQ_WARPS * 32, 4) k_ccd_ee(
     BvhSet bv, const CcdPass* __restrict__ cpp, const uint8_t* __restrict__ vinst, const float* __restrict__ x,
     const float* __restrict__ dx, const uint32_t* __restrict__ edges, const uint32_t* __restrict__ ee_tail,
     const float* __restrict__ im, uint32_t ne, uint32_t max_iter, unsigned int* __restrict__ red,
-    unsigned int* __restrict__ acc, uint32_t* __restrict__ status) {
-  __shared__ uint2 qbuf[WQ_WARPS][WQ_QCAP];
-  uint2* q = qbuf[threadIdx.x >> 5];
-  int qn = 0;
+    unsigned int* __restrict__ acc, uint32_t* __restrict__ status, uint32_t per) {
+  __shared__ WalkMem<CcdQuery> mem[WQ_WARPS];
   const CcdPass& cp = *cpp;
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t k = 0xffffffffu, base = 0, nleaf = 0;
-  bool done = true;
-  CcdWalk walk;
-  walk.ok = true;
-  uint32_t out[2];
-  int nout = 0;
-  if (j < ne) {
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, first = (blockIdx.x * WQ_WARPS + w) * per;
+  const uint32_t j = first + lane;
+  CcdQuery q;
+  uint32_t k = 0;
+  bool valid = false;
+  if (lane < per && j < ne) {
     const uint32_t b0 = edges[2 * j], b1 = edges[2 * j + 1];
-    const uint32_t kj = vinst[b0];
-    if (((cp.todo >> kj) & 1u) && j < ee_tail[kj]) {
-      k = kj;
-      base = bv.base[k];
-      float4 lo, hi, qlo, qhi;
-      edge_box(x, b0, b1, cp.search[k][cp.npass[k] - 1], lo, hi);
-      edge_box(x, b0, b1, 0.f, qlo, qhi);
+    k = vinst[b0];
+    valid = ((cp.todo >> k) & 1u) && j < ee_tail[k];
+    if (valid) {
+      edge_box(x, b0, b1, cp.search[k][cp.npass[k] - 1], q.slo, q.shi);
+      edge_box(x, b0, b1, 0.f, q.qlo, q.qhi);
       // the query edge's displacements lie in the ball around their midpoint
       const float3 d0 = make_float3(dx[3 * b0], dx[3 * b0 + 1], dx[3 * b0 + 2]);
       const float3 d1 = make_float3(dx[3 * b1], dx[3 * b1 + 1], dx[3 * b1 + 2]);
-      const float3 cq = make_float3(0.5f * (d0.x + d1.x), 0.5f * (d0.y + d1.y), 0.5f * (d0.z + d1.z));
       const float ex = d1.x - d0.x, ey = d1.y - d0.y, ez = d1.z - d0.z;
-      const float rq = 0.5f * sqrtf(ex * ex + ey * ey + ez * ez) * 1.0001f;
-      walk_init(walk, bv, k, lo, hi, qlo, qhi, cq, rq);
-      nout = walk.start(done, out);
+      q.c = make_float4(0.5f * (d0.x + d1.x), 0.5f * (d0.y + d1.y), 0.5f * (d0.z + d1.z),
+                        0.5f * sqrtf(ex * ex + ey * ey + ez * ez) * 1.0001f);
     }
   }
+  LeafCount nleaf{0u, 0u, red, 7};
   CcdAcc a;
   a.reset(0xffffffffu);
   auto solve = [&](uint2 e) {
@@ -877,22 +929,13 @@ __global__ void __launch_bounds__(WQ_WARPS * 32, 4) k_ccd_ee(
     const R toi = accd_toi<R>(x0, dd, R(0), R(1.25), R(0.01), max_iter, 1, &capped);
     a.add(kq, i0, (float)(toi / R(1.25)), capped, cp, acc, red, 8);
   };
-  for (;;) {
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const bool leaf = c < nout;
-      const uint32_t i = leaf ? base + out[c] : 0u;
-      nleaf += leaf ? 1u : 0u;
-      wq_push(q, qn, leaf && i > j, make_uint2(j, i));
-    }
-    wq_take(q, qn, 32, solve);
-    if (!__any_sync(0xffffffffu, !done)) break;
-    nout = done ? 0 : walk.step(done, out);
-  }
-  wq_take(q, qn, 1, solve);
+  auto keep = [&](uint32_t slot, uint32_t i) {
+    nleaf.add(mem[w].inst[slot]);
+    return i > first + slot;
+  };
+  if (!warp_walk(mem[w], bv, first, valid, k, q, keep, solve)) atomicOr(status, ST_STACK_OVERFLOW);
   a.flush(cp, acc, red, 8);
-  if (!walk.ok) atomicOr(status, ST_STACK_OVERFLOW);
-  if (nleaf) atomicAdd(red + RED_STRIDE * k + 7, nleaf);
+  nleaf.flush();
 }
 
 // ccd_max_step (implicit.rs:1690-1947) without strain limiting, per instance. The
@@ -1025,23 +1068,16 @@ static void ccd_body(Scene& s, const BvhSet& tv, const BvhSet& ev, CcdState* cs)
   const uint32_t iters = std::max<uint32_t>(s.p.ccd_max_iter, 1);
   const CcdPass* cpp = &cs->cp;
   k_ccd_plan<<<1, PCG_MAX_INST * CCD_CHUNK, 0, st>>>(cs, s.ccd_acc.p, fixed);
-  if (s.mixed) {
-    k_ccd_vt<double><<<ceil_div(s.nv, 128), 128, 0, st>>>(
-        tv, cpp, s.vinst.p, s.x.p, s.dx.p, s.tris.p, s.collider_tri.p, s.inv_mass.p, s.ex_ptr.p, s.ex_list.p,
-        s.side_best.p, s.collider_pn.p, s.has_static ? 1 : 0, s.nv, dhat, iters, s.red.p, s.ccd_acc.p, s.status.p);
-    if (s.n_edge)
-      k_ccd_ee<double><<<ceil_div(s.n_edge, 128), 128, 0, st>>>(ev, cpp, s.vinst.p, s.x.p, s.dx.p, s.edges.p,
-                                                               s.ee_tail.p, s.inv_mass.p, s.n_edge, iters, s.red.p, s.ccd_acc.p,
-                                                               s.status.p);
-  } else {
-    k_ccd_vt<float><<<ceil_div(s.nv, 128), 128, 0, st>>>(
-        tv, cpp, s.vinst.p, s.x.p, s.dx.p, s.tris.p, s.collider_tri.p, s.inv_mass.p, s.ex_ptr.p, s.ex_list.p,
-        s.side_best.p, s.collider_pn.p, s.has_static ? 1 : 0, s.nv, dhat, iters, s.red.p, s.ccd_acc.p, s.status.p);
-    if (s.n_edge)
-      k_ccd_ee<float><<<ceil_div(s.n_edge, 128), 128, 0, st>>>(ev, cpp, s.vinst.p, s.x.p, s.dx.p, s.edges.p,
-                                                              s.ee_tail.p, s.inv_mass.p, s.n_edge, iters, s.red.p, s.ccd_acc.p,
-                                                              s.status.p);
-  }
+  const uint32_t vper = walk_per(s, s.nv), eper = walk_per(s, s.n_edge);
+  const uint32_t vg = walk_grid(s.nv, vper), eg = walk_grid(s.n_edge, eper);
+  auto vt = s.mixed ? k_ccd_vt<double> : k_ccd_vt<float>;
+  auto ee = s.mixed ? k_ccd_ee<double> : k_ccd_ee<float>;
+  vt<<<vg, WQ_WARPS * 32, 0, st>>>(tv, cpp, s.vinst.p, s.x.p, s.dx.p, s.tris.p, s.collider_tri.p, s.inv_mass.p,
+                                   s.ex_ptr.p, s.ex_list.p, s.side_best.p, s.collider_pn.p, s.has_static ? 1 : 0, s.nv,
+                                   dhat, iters, s.red.p, s.ccd_acc.p, s.status.p, vper);
+  if (s.n_edge)
+    ee<<<eg, WQ_WARPS * 32, 0, st>>>(ev, cpp, s.vinst.p, s.x.p, s.dx.p, s.edges.p, s.ee_tail.p, s.inv_mass.p, s.n_edge,
+                                     iters, s.red.p, s.ccd_acc.p, s.status.p, eper);
 }
 
 // The self-contact schedule's graph: one conditional while node around plan, the two

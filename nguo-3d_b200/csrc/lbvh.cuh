@@ -68,222 +68,45 @@ struct mguso_lbvh {
 
 namespace mg {
 
-// Visits every leaf whose box overlaps [qlo, qhi] (the predicate of
-// bvh_traverse.wgsl:64-92), calling f(leaf_primitive). 64-entry stack; returns false on
-// stack overflow.
-template <class F>
-__device__ __forceinline__ bool lbvh_visit(const uint32_t* __restrict__ left, const uint32_t* __restrict__ right,
-                                           const float4* __restrict__ node, const float4* __restrict__ leaf,
-                                           const uint32_t* __restrict__ prim, uint32_t nt, float4 qlo, float4 qhi,
-                                           F&& f) {
-  auto ov = [&](const float4& lo, const float4& hi) {
-    return qlo.x <= hi.x && qlo.y <= hi.y && qlo.z <= hi.z && lo.x <= qhi.x && lo.y <= qhi.y && lo.z <= qhi.z;
-  };
-  if (nt == 0) return true;
-  if (nt == 1) {
-    if (ov(leaf[0], leaf[1])) f(prim[0]);
-    return true;
-  }
-  if (!ov(__ldg(node), __ldg(node + 1))) return true;
-  uint32_t stack[64];
-  int sp = 0;
-  uint32_t cur = 0;
-  bool ok = true;
-  for (;;) {
-    uint32_t ch[2] = {__ldg(left + cur), __ldg(right + cur)};
-    uint32_t next = 0xffffffffu;
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      uint32_t x = ch[c];
-      const float4* b = (x & 0x80000000u) ? leaf + 2 * (x & 0x7fffffffu) : node + 2 * x;
-      if (!ov(__ldg(b), __ldg(b + 1))) continue;
-      if (x & 0x80000000u) {
-        f(prim[x & 0x7fffffffu]);
-      } else if (next == 0xffffffffu) {
-        next = x;
-      } else if (sp < 64) {
-        stack[sp++] = x;
-      } else {
-        ok = false;
-      }
-    }
-    if (next != 0xffffffffu) {
-      cur = next;
-    } else if (sp > 0) {
-      cur = stack[--sp];
-    } else {
-      break;
-    }
-  }
-  return ok;
+__device__ __forceinline__ bool boxes_overlap(const float4& qlo, const float4& qhi, const float4& lo, const float4& hi) {
+  return qlo.x <= hi.x && qlo.y <= hi.y && qlo.z <= hi.z && lo.x <= qhi.x && lo.y <= qhi.y && lo.z <= qhi.z;
 }
 
-// Resumable walk over the leaves whose boxes overlap [qlo, qhi] (the predicate of
-// lbvh_visit): start() and each step() hand back at most two leaf primitives, so a warp's
-// lanes can advance their walks in lockstep and pool the leaves they reach. 64-entry stack;
-// ok turns false on overflow.
-struct BoxWalk {
-  const uint32_t *left, *right, *prim;
-  const float4 *node, *leaf, *cbox;
-  uint32_t nt;
-  float4 qlo, qhi;
-  uint32_t stack[64];
-  int sp;
-  uint32_t cur;
-  bool ok;
-
-  __device__ __forceinline__ bool over(const float4& lo, const float4& hi) const {
-    return qlo.x <= hi.x && qlo.y <= hi.y && qlo.z <= hi.z && lo.x <= qhi.x && lo.y <= qhi.y && lo.z <= qhi.z;
-  }
-  __device__ __forceinline__ bool enter(const float4* pb) const { return over(__ldg(pb), __ldg(pb + 1)); }
-  __device__ __forceinline__ int start(bool& done, uint32_t out[2]) {
-    sp = 0;
-    cur = 0;
-    ok = true;
-    done = true;
-    if (nt == 0) return 0;
-    if (nt == 1) {
-      if (enter(leaf)) {
-        out[0] = prim[0];
-        return 1;
-      }
-      return 0;
-    }
-    done = !enter(node);
-    return 0;
-  }
-  __device__ __forceinline__ int step(bool& done, uint32_t out[2]) {
-    int n = 0;
-    const uint32_t ch[2] = {__ldg(left + cur), __ldg(right + cur)};
-    const float4* cb = cbox + 4 * (size_t)cur;
-    const bool in[2] = {over(__ldg(cb), __ldg(cb + 1)), over(__ldg(cb + 2), __ldg(cb + 3))};
-    uint32_t next = 0xffffffffu;
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const uint32_t x = ch[c];
-      const bool lf = (x & 0x80000000u) != 0;
-      const uint32_t i = x & 0x7fffffffu;
-      if (!in[c]) continue;
-      if (lf) {
-        out[n++] = prim[i];
-      } else if (next == 0xffffffffu) {
-        next = x;
-      } else if (sp < 64) {
-        stack[sp++] = x;
-      } else {
-        ok = false;
-      }
-    }
-    if (next != 0xffffffffu) {
-      cur = next;
-    } else if (sp > 0) {
-      cur = stack[--sp];
-    } else {
-      done = true;
-    }
-    return n;
-  }
-};
-
-// CCD traversal (ccd_max_step's broad phase, implicit.rs:1690-1947, with exact pruning).
-// A subtree is entered when the search box overlaps its position box (node, leaf) and its
+// CCD traversal test (ccd_max_step's broad phase, implicit.rs:1690-1947, with exact pruning).
+// A subtree is entered when the search box overlaps its position box [lo, hi] and its
 // pairs with the query are not all settled by accd_toi's first test (contact.rs:378-437),
 // which returns max_t = 1.25 whenever 1.25 u_max < 0.98 d0 (u_max: the largest relative
 // displacement of the pair's four points; d0: their distance). Over a subtree, with the
 // query's displacements inside the ball (cq, rq) and the subtree's inside its displacement
-// box D (dnode, dleaf), the pairs' relative displacements are bounded by 2 rq (within the
-// query), the diagonal of D (within a primitive) and rq + farthest(cq, D) (across), so
-// u_max <= max(2 rq, diag D, rq + farthest(cq, D)); and d0 >= the distance between the
-// query's box (qlo, qhi) and the subtree's position box. The subtree is skipped when
-// 1.3 u_bound < 0.98 distance (4% margin over 1.25 for rounding).
-//
-// The walk is resumable: start() and each step() hand back at most two leaf primitives, so
-// the lanes of a warp can advance their walks in lockstep and pool the leaves they reach
-// (the root solves then run on full warps). 64-entry stack; ok turns false on overflow.
-struct CcdWalk {
-  const uint32_t *left, *right, *prim;
-  const float4 *node, *leaf, *dnode, *dleaf, *cbox, *dcbox;
-  uint32_t nt;
+// box D (db, read only when needed), the pairs' relative displacements are bounded by 2 rq
+// (within the query), the diagonal of D (within a primitive) and rq + farthest(cq, D)
+// (across), so u_max <= max(2 rq, diag D, rq + farthest(cq, D)); and d0 >= the distance
+// between the query's box (qlo, qhi) and the subtree's position box. The subtree is skipped
+// when 1.3 u_bound < 0.98 distance (4% margin over 1.25 for rounding).
+struct CcdQuery {
   float4 slo, shi, qlo, qhi;
-  float3 cq;
-  float rq;
-  uint32_t stack[64];
-  int sp;
-  uint32_t cur;
-  bool ok;
-
-  __device__ __forceinline__ bool enter(const float4* pb, const float4* db) const {
-    return enter_box(__ldg(pb), __ldg(pb + 1), db);
-  }
-  // the test of enter() with the position box given (db: the displacement box, read only
-  // when the pruning bound is needed)
-  __device__ __forceinline__ bool enter_box(const float4 lo, const float4 hi, const float4* db) const {
-    if (!(slo.x <= hi.x && slo.y <= hi.y && slo.z <= hi.z && lo.x <= shi.x && lo.y <= shi.y && lo.z <= shi.z))
-      return false;
+  float4 c;  // cq, rq
+  __device__ __forceinline__ bool enter(const float4 lo, const float4 hi, const float4* db) const {
+    if (!boxes_overlap(slo, shi, lo, hi)) return false;
     const float gx = fmaxf(fmaxf(qlo.x - hi.x, lo.x - qhi.x), 0.f);
     const float gy = fmaxf(fmaxf(qlo.y - hi.y, lo.y - qhi.y), 0.f);
     const float gz = fmaxf(fmaxf(qlo.z - hi.z, lo.z - qhi.z), 0.f);
     const float gap2 = gx * gx + gy * gy + gz * gz;
     if (gap2 == 0.f) return true;
     const float4 dlo = __ldg(db), dhi = __ldg(db + 1);
-    const float fx = fmaxf(fabsf(cq.x - dlo.x), fabsf(cq.x - dhi.x));
-    const float fy = fmaxf(fabsf(cq.y - dlo.y), fabsf(cq.y - dhi.y));
-    const float fz = fmaxf(fabsf(cq.z - dlo.z), fabsf(cq.z - dhi.z));
+    const float rq = c.w;
+    const float fx = fmaxf(fabsf(c.x - dlo.x), fabsf(c.x - dhi.x));
+    const float fy = fmaxf(fabsf(c.y - dlo.y), fabsf(c.y - dhi.y));
+    const float fz = fmaxf(fabsf(c.z - dlo.z), fabsf(c.z - dhi.z));
     const float ex = dhi.x - dlo.x, ey = dhi.y - dlo.y, ez = dhi.z - dlo.z;
     const float u = fmaxf(fmaxf(2.f * rq, sqrtf(ex * ex + ey * ey + ez * ez)), rq + sqrtf(fx * fx + fy * fy + fz * fz));
     return !(1.3f * u < 0.98f * sqrtf(gap2));
   }
-  // Begins the walk; returns the number of leaves written to out (the single leaf of a
-  // one-primitive tree) and sets done when nothing is left to visit.
-  __device__ __forceinline__ int start(bool& done, uint32_t out[2]) {
-    sp = 0;
-    cur = 0;
-    ok = true;
-    done = true;
-    if (nt == 0) return 0;
-    if (nt == 1) {
-      if (enter(leaf, dleaf)) {
-        out[0] = prim[0];
-        return 1;
-      }
-      return 0;
-    }
-    done = !enter(node, dnode);
-    return 0;
-  }
-  // Visits the children of the current node: entered leaves go to out (returned count),
-  // an entered inner child becomes the next node (the second is stacked).
-  __device__ __forceinline__ int step(bool& done, uint32_t out[2]) {
-    int n = 0;
-    const uint32_t ch[2] = {__ldg(left + cur), __ldg(right + cur)};
-    const float4* cb = cbox + 4 * (size_t)cur;
-    const float4* db = dcbox + 4 * (size_t)cur;
-    const bool in[2] = {enter_box(__ldg(cb), __ldg(cb + 1), db), enter_box(__ldg(cb + 2), __ldg(cb + 3), db + 2)};
-    uint32_t next = 0xffffffffu;
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const uint32_t x = ch[c];
-      const bool lf = (x & 0x80000000u) != 0;
-      const uint32_t i = x & 0x7fffffffu;
-      if (!in[c]) continue;
-      if (lf) {
-        out[n++] = prim[i];
-      } else if (next == 0xffffffffu) {
-        next = x;
-      } else if (sp < 64) {
-        stack[sp++] = x;
-      } else {
-        ok = false;
-      }
-    }
-    if (next != 0xffffffffu) {
-      cur = next;
-    } else if (sp > 0) {
-      cur = stack[--sp];
-    } else {
-      done = true;
-    }
-    return n;
+};
+struct BoxQuery {
+  float4 lo, hi;
+  __device__ __forceinline__ bool enter(const float4 blo, const float4 bhi, const float4*) const {
+    return boxes_overlap(lo, hi, blo, bhi);
   }
 };
 
