@@ -192,7 +192,7 @@ int mguso_radix_sort_status(mguso_ctx* ctx);
  * For callers that may not allocate device memory once they are running (a host engine
  * that gives all of the GPU's memory to its own pool at start-up, or a per-frame path that
  * cannot afford cudaMalloc's device-wide synchronisation): it allocates nothing and needs
- * no context. Its temporaries live in one fixed 3.2 MiB device array inside this library
+ * no context. Its temporaries live in one fixed 4.1 MiB device array inside this library
  * (on every device that loads it, until the process exits), which limits n to 262 144
  * pairs; larger n returns MGUSO_ERR_INVALID_ARG. Sorts the same (key, payload) pairs in
  * place on the current device, stably, with the same result as mguso_radix_sort_pairs, and

@@ -137,84 +137,87 @@ __global__ void k_morton_points(const float* __restrict__ pts, uint32_t np, cons
 // ---------------------------------------------------------------------------------------
 // Onesweep radix sort (stable LSD, 8-bit digits, decoupled look-back across tiles)
 // ---------------------------------------------------------------------------------------
-constexpr int RS_THREADS = 256;
-constexpr int RS_WARPS = RS_THREADS / 32;
-constexpr int RS_ITEMS = 8;
-constexpr uint32_t RS_TILE = RS_THREADS * RS_ITEMS;  // 2048 keys per tile
+// Tiles: a pass is bound by latency when it has few tiles (ranking, then the look-back) and by the
+// scatter's short runs and the look-back's chain when it has many. Small sorts take tiles of 2 048
+// keys, so that 65 536 keys still spread over 32 SMs; from RS_LARGE keys on tiles of 6 144, whose
+// runs per digit are three times as long. A pass over 65 536 u32 keys before -> after
+// (look-back words read eight at a time, one memset for all passes, the digit scan in the pass
+// itself): 9.8 -> 8.3 us, with half the launches between (whole sort 79 -> 53 us); a pass over
+// 4 M keys and one over 12.6 M together 270 -> 199 us.
+constexpr uint32_t RS_TILE_S = 256 * 8, RS_TILE_L = 384 * 16;
+constexpr uint32_t RS_LARGE = 1u << 20;
 constexpr uint32_t FLAG_AGG = 1u << 30, FLAG_PRE = 2u << 30, VAL_MASK = (1u << 30) - 1;
+constexpr int RS_LOOK = 8;  // predecessors read at once by the look-back
 
 template <class K>
-__global__ void k_rs_hist(const K* __restrict__ keys, uint32_t n, int passes, uint32_t* __restrict__ hist) {
+__global__ void __launch_bounds__(256) k_rs_hist(const K* __restrict__ keys, uint32_t n, int passes,
+                                                 uint32_t* __restrict__ hist) {
   __shared__ uint32_t sh[8 * 256];
   for (int i = threadIdx.x; i < passes * 256; i += blockDim.x) sh[i] = 0;
   __syncthreads();
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    K k = keys[i];
-    for (int p = 0; p < passes; ++p) atomicAdd(&sh[p * 256 + (uint32_t)((k >> (8 * p)) & 0xff)], 1u);
+  const uint32_t st = gridDim.x * blockDim.x;
+  for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 4 * st) {
+    K k[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) k[u] = i0 + u * (uint64_t)st < n ? keys[i0 + u * st] : (K)0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i0 + u * (uint64_t)st < n)
+        for (int p = 0; p < passes; ++p) atomicAdd(&sh[p * 256 + (uint32_t)((k[u] >> (8 * p)) & 0xff)], 1u);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < passes * 256; i += blockDim.x)
     if (sh[i]) atomicAdd(&hist[i], sh[i]);
 }
 
-// exclusive scan of each pass's 256 counts (one CTA of 256 threads per pass)
-__global__ void k_rs_scan(const uint32_t* __restrict__ hist, uint32_t* __restrict__ ofs) {
-  __shared__ uint32_t s[256];
-  int p = blockIdx.x, d = threadIdx.x;
-  uint32_t v = hist[p * 256 + d];
-  s[d] = v;
-  __syncthreads();
-  for (int o = 1; o < 256; o <<= 1) {
-    uint32_t t = d >= o ? s[d - o] : 0;
-    __syncthreads();
-    s[d] += t;
-    __syncthreads();
-  }
-  ofs[p * 256 + d] = s[d] - v;
-}
-
-template <class K>
-__global__ void __launch_bounds__(RS_THREADS) k_onesweep(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
-                                                         K* __restrict__ kout, uint32_t* __restrict__ vout,
-                                                         uint32_t n, int shift, const uint32_t* __restrict__ gofs,
-                                                         uint32_t* status, uint32_t* tile_counter, uint32_t* err,
-                                                         const uint32_t* __restrict__ phist) {
-  // phist (the pass's digit histogram, or null): when every key has the same digit the pass
-  // keeps the order, and each CTA only copies its tile (the same decision in every CTA, so
-  // no look-back is started); the host then never reads the histogram back
-  if (phist && phist[(uint32_t)((kin[0] >> shift) & 0xff)] == n) {
-    const uint32_t b0 = blockIdx.x * RS_TILE, b1 = min(b0 + RS_TILE, n);
-    for (uint32_t j = b0 + threadIdx.x; j < b1; j += RS_THREADS) {
+// One pass: phist is its digit histogram, `skip` whether a pass whose keys all have one digit
+// may only copy (the same decision in every CTA, so no look-back is started; the host never
+// reads the histogram back).
+template <class K, int THREADS, int ITEMS>
+__global__ void __launch_bounds__(THREADS) k_onesweep(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
+                                                      K* __restrict__ kout, uint32_t* __restrict__ vout, uint32_t n,
+                                                      int shift, const uint32_t* __restrict__ phist, int skip,
+                                                      uint32_t* status, uint32_t* tile_counter, uint32_t* err) {
+  constexpr uint32_t TILE = THREADS * ITEMS;
+  constexpr int WARPS = THREADS / 32;
+  extern __shared__ __align__(16) unsigned char rs_smem[];
+  K* skeys = reinterpret_cast<K*>(rs_smem);
+  uint32_t* svals = reinterpret_cast<uint32_t*>(skeys + TILE);
+  __shared__ uint32_t whist[WARPS][256];
+  __shared__ uint32_t tile_excl[256], g_pref[256];
+  __shared__ uint32_t wsum[8], gsum[8];
+  __shared__ uint32_t s_tile;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  if (skip && phist[(uint32_t)((kin[0] >> shift) & 0xff)] == n) {
+    const uint32_t b0 = blockIdx.x * TILE, b1 = min(b0 + TILE, n);
+    for (uint32_t j = b0 + tid; j < b1; j += THREADS) {
       kout[j] = kin[j];
       vout[j] = vin[j];
     }
     return;
   }
-  __shared__ uint32_t whist[RS_WARPS][256];
-  __shared__ uint32_t tile_excl[256], g_pref[256];
-  __shared__ K skeys[RS_TILE];
-  __shared__ uint32_t svals[RS_TILE];
-  __shared__ uint32_t s_tile;
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   if (tid == 0) s_tile = atomicAdd(tile_counter, 1u);
   for (int d = lane; d < 256; d += 32) whist[w][d] = 0;
   __syncthreads();
   const uint32_t tile = s_tile;
-  const uint32_t base = tile * RS_TILE;
-  const uint32_t tile_n = min(RS_TILE, n - base);
-  K key[RS_ITEMS];
-  uint32_t val[RS_ITEMS], rank[RS_ITEMS];
-  const uint32_t wbase = base + (uint32_t)w * RS_ITEMS * 32;
+  const uint32_t base = tile * TILE;
+  const uint32_t tile_n = min(TILE, n - base);
+  K key[ITEMS];
+  uint32_t val[ITEMS], rank[ITEMS];
+  const uint32_t wbase = base + (uint32_t)w * ITEMS * 32;
 #pragma unroll
-  for (int i = 0; i < RS_ITEMS; ++i) {
-    uint32_t idx = wbase + i * 32 + lane;
-    bool valid = idx < n;
-    key[i] = valid ? kin[idx] : (K)0;
-    val[i] = valid ? vin[idx] : 0u;
-    uint32_t d = valid ? (uint32_t)((key[i] >> shift) & 0xff) : 0x100u + lane;
-    uint32_t peers = __match_any_sync(0xffffffffu, d);
-    int leader = __ffs(peers) - 1;
-    uint32_t before = __popc(peers & ((1u << lane) - 1u));
+  for (int i = 0; i < ITEMS; ++i) {
+    const uint32_t idx = wbase + i * 32 + lane;
+    key[i] = idx < n ? kin[idx] : (K)0;
+    val[i] = idx < n ? vin[idx] : 0u;
+  }
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) {
+    const bool valid = wbase + i * 32 + lane < n;
+    const uint32_t d = valid ? (uint32_t)((key[i] >> shift) & 0xff) : 0x100u + lane;
+    const uint32_t peers = __match_any_sync(0xffffffffu, d);
+    const int leader = __ffs(peers) - 1;
+    const uint32_t before = __popc(peers & ((1u << lane) - 1u));
     uint32_t old = 0;
     if (valid && lane == leader) {
       old = whist[w][d];
@@ -225,73 +228,84 @@ __global__ void __launch_bounds__(RS_THREADS) k_onesweep(const K* __restrict__ k
     __syncwarp();
   }
   __syncthreads();
-  // per digit: offsets of each warp, tile count, look-back for the global prefix
-  {
+  // per digit: offsets of each warp, the tile's count (published), and, while that travels, the
+  // digit's start in the tile and in the whole output
+  uint32_t run = 0, tincl = 0, gincl = 0, gcount = 0;
+  if (tid < 256) {
     const int d = tid;
-    uint32_t run = 0;
-    for (int ww = 0; ww < RS_WARPS; ++ww) {
-      uint32_t c = whist[ww][d];
+    for (int ww = 0; ww < WARPS; ++ww) {
+      const uint32_t c = whist[ww][d];
       whist[ww][d] = run;
       run += c;
     }
-    volatile uint32_t* st = status;
-    st[(size_t)tile * 256 + d] = FLAG_AGG | run;
-    uint32_t excl = 0;
-    int64_t j = (int64_t)tile - 1;
-    uint32_t spins = 0;
-    while (j >= 0) {
-      uint32_t v = st[(size_t)j * 256 + d];
-      uint32_t flag = v & ~VAL_MASK;
-      if (flag == 0) {
-        if (++spins > (1u << 26)) {
-          atomicOr(err, ST_WAIT_TIMEOUT);
-          break;
-        }
-        continue;
+    ((volatile uint32_t*)status)[(size_t)tile * 256 + d] = (tile ? FLAG_AGG : FLAG_PRE) | run;
+    gcount = phist[d];
+    tincl = run;
+    gincl = gcount;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, tincl, o), g = __shfl_up_sync(0xffffffffu, gincl, o);
+      if (lane >= o) {
+        tincl += t;
+        gincl += g;
       }
-      excl += v & VAL_MASK;
-      if (flag == FLAG_PRE) break;
-      --j;
     }
-    __threadfence();
-    st[(size_t)tile * 256 + d] = FLAG_PRE | (excl + run);
-    g_pref[d] = gofs[d] + excl;
-    tile_excl[d] = run;  // scanned below
+    if (lane == 31) {
+      wsum[w] = tincl;
+      gsum[w] = gincl;
+    }
   }
   __syncthreads();
-  // exclusive scan of the tile's digit counts (256 entries, one per thread)
-  {
+  if (tid < 256) {
     const int d = tid;
-    uint32_t v = tile_excl[d];
-    uint32_t incl = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
+    uint32_t tofs = 0, gofs = 0;
+    for (int ww = 0; ww < w; ++ww) {
+      tofs += wsum[ww];
+      gofs += gsum[ww];
     }
-    __shared__ uint32_t wsum[RS_WARPS];
-    if (lane == 31) wsum[w] = incl;
-    __syncthreads();
-    uint32_t wofs = 0;
-    for (int ww = 0; ww < w; ++ww) wofs += wsum[ww];
-    __syncthreads();
-    tile_excl[d] = wofs + incl - v;
+    tile_excl[d] = tofs + tincl - run;
+    // decoupled look-back, RS_LOOK predecessors in flight
+    uint32_t excl = 0, spins = 0;
+    int64_t j = (int64_t)tile - 1;
+    bool more = tile > 0;
+    while (more) {
+      uint32_t v[RS_LOOK];
+#pragma unroll
+      for (int u = 0; u < RS_LOOK; ++u)
+        v[u] = j - u >= 0 ? ((volatile uint32_t*)status)[(size_t)(j - u) * 256 + d] : FLAG_PRE + 0u;
+      int used = 0;
+#pragma unroll
+      for (int u = 0; u < RS_LOOK; ++u) {
+        if (!more || used < u) continue;  // stopped at an earlier one
+        const uint32_t flag = v[u] & ~VAL_MASK;
+        if (flag == 0) continue;
+        used = u + 1;
+        excl += v[u] & VAL_MASK;
+        if (flag == FLAG_PRE) more = false;
+      }
+      j -= used;
+      if (used == 0 && ++spins > (1u << 24)) {
+        atomicOr(err, ST_WAIT_TIMEOUT);
+        break;
+      }
+    }
+    if (tile) ((volatile uint32_t*)status)[(size_t)tile * 256 + d] = FLAG_PRE | (excl + run);
+    g_pref[d] = gofs + gincl - gcount + excl;
   }
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < RS_ITEMS; ++i) {
-    uint32_t idx = wbase + i * 32 + lane;
-    if (idx < n) {
-      uint32_t d = (uint32_t)((key[i] >> shift) & 0xff);
-      uint32_t p = tile_excl[d] + whist[w][d] + rank[i];
+  for (int i = 0; i < ITEMS; ++i) {
+    if (wbase + i * 32 + lane < n) {
+      const uint32_t d = (uint32_t)((key[i] >> shift) & 0xff);
+      const uint32_t p = tile_excl[d] + whist[w][d] + rank[i];
       skeys[p] = key[i];
       svals[p] = val[i];
     }
   }
   __syncthreads();
-  for (uint32_t j = tid; j < tile_n; j += RS_THREADS) {
-    K k = skeys[j];
-    uint32_t d = (uint32_t)((k >> shift) & 0xff);
-    uint32_t o = g_pref[d] + (j - tile_excl[d]);
+  for (uint32_t j = tid; j < tile_n; j += THREADS) {
+    const K k = skeys[j];
+    const uint32_t d = (uint32_t)((k >> shift) & 0xff);
+    const uint32_t o = g_pref[d] + (j - tile_excl[d]);
     kout[o] = k;
     vout[o] = svals[j];
   }
@@ -503,35 +517,57 @@ __global__ void __launch_bounds__(128) k_traverse(const uint32_t* __restrict__ l
 // ---------------------------------------------------------------------------------------
 // Host orchestration
 // ---------------------------------------------------------------------------------------
-template <class K>
-static int sort_impl(Lbvh* b, K* keys, uint32_t* vals, uint32_t n, int key_bits, cudaStream_t s) {
-  if (n <= 1) return MGUSO_OK;
-  int passes = (key_bits + 7) / 8;
-  MG_TRY(b->rs_hist.reserve(8 * 256));
-  MG_TRY(b->rs_ofs.reserve(8 * 256));
-  uint32_t ntiles = ceil_div(n, RS_TILE);
-  MG_TRY(b->rs_status.grow((size_t)ntiles * 256));
-  MG_TRY(b->rs_counter.reserve(8));
-  MG_TRY(b->rs_tmpk.grow((size_t)n * sizeof(K)));
-  MG_TRY(b->rs_tmpv.grow(n));
-  MG_CUDA(cudaMemsetAsync(b->rs_hist.p, 0, 4 * 8 * 256, s));
-  int sms = device_sm_count();
-  k_rs_hist<K><<<std::min<uint32_t>(ceil_div(n, 256), sms * 8), 256, 0, s>>>(keys, n, passes, b->rs_hist.p);
-  k_rs_scan<<<passes, 256, 0, s>>>(b->rs_hist.p, b->rs_ofs.p);
+// The sort's device scratch: digit histograms of all passes, a tile counter per pass and the
+// look-back words of all passes, laid out in that order so that one memset clears them.
+struct SortScratch {
+  uint32_t* words;
+  unsigned char* tmpk;
+  uint32_t *tmpv, *err;
+};
+static uint32_t rs_tile(uint32_t n) { return n >= RS_LARGE ? RS_TILE_L : RS_TILE_S; }
+static size_t rs_words(uint32_t n, int passes) {
+  return (size_t)passes * (256 + 1 + (size_t)ceil_div(n, rs_tile(n)) * 256);
+}
+
+template <class K, int THREADS, int ITEMS>
+static int sort_pass(const K* kA, const uint32_t* vA, K* kB, uint32_t* vB, uint32_t n, int shift, const uint32_t* hist,
+                     int skip, uint32_t* status, uint32_t* counter, uint32_t* err, cudaStream_t s) {
+  constexpr uint32_t TILE = THREADS * ITEMS;
+  constexpr int smem = (int)(TILE * (sizeof(K) + 4));
+  auto fn = k_onesweep<K, THREADS, ITEMS>;
+  if (smem > 32 * 1024) MG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  fn<<<ceil_div(n, TILE), THREADS, smem, s>>>(kA, vA, kB, vB, n, shift, hist, skip, status, counter, err);
   MG_CUDA(cudaGetLastError());
-  // every pass is launched; a pass whose digit is the same for every key finds that out on
-  // the device and only copies, so the sort needs no readback
+  return MGUSO_OK;
+}
+
+// Every pass is launched; with `skip`, a pass whose digit is the same for every key finds that
+// out on the device and only copies, so the sort needs no readback.
+template <class K>
+static int sort_run(const SortScratch& sc, K* keys, uint32_t* vals, uint32_t n, int key_bits, int skip,
+                    cudaStream_t s) {
+  const int passes = (key_bits + 7) / 8;
+  const uint32_t ntiles = ceil_div(n, rs_tile(n));
+  uint32_t* hist = sc.words;
+  uint32_t* counter = hist + 256 * passes;
+  uint32_t* status = counter + passes;
+  MG_CUDA(cudaMemsetAsync(sc.words, 0, 4 * rs_words(n, passes), s));
+  const int sms = device_sm_count();
+  k_rs_hist<K><<<std::min<uint32_t>(ceil_div(n, 1024), sms * 8), 256, 0, s>>>(keys, n, passes, hist);
+  MG_CUDA(cudaGetLastError());
   K* kA = keys;
   uint32_t* vA = vals;
-  K* kB = (K*)b->rs_tmpk.p;
-  uint32_t* vB = b->rs_tmpv.p;
+  K* kB = (K*)sc.tmpk;
+  uint32_t* vB = sc.tmpv;
   for (int p = 0; p < passes; ++p) {
-    MG_CUDA(cudaMemsetAsync(b->rs_status.p, 0, 4 * (size_t)ntiles * 256, s));
-    MG_CUDA(cudaMemsetAsync(b->rs_counter.p, 0, 4, s));
-    k_onesweep<K><<<ntiles, RS_THREADS, 0, s>>>(kA, vA, kB, vB, n, 8 * p, b->rs_ofs.p + p * 256, b->rs_status.p,
-                                               b->rs_counter.p, b->err_sink ? b->err_sink : b->status.p,
-                                               b->rs_hist.p + p * 256);
-    MG_CUDA(cudaGetLastError());
+    const auto args = [&](auto fn) {
+      return fn(kA, vA, kB, vB, n, 8 * p, hist + 256 * p, skip, status + (size_t)p * ntiles * 256, counter + p, sc.err,
+                s);
+    };
+    if (n >= RS_LARGE)
+      MG_TRY(args(sort_pass<K, 384, 16>));
+    else
+      MG_TRY(args(sort_pass<K, 256, 8>));
     std::swap(kA, kB);
     std::swap(vA, vB);
   }
@@ -540,6 +576,16 @@ static int sort_impl(Lbvh* b, K* keys, uint32_t* vals, uint32_t n, int key_bits,
     MG_CUDA(cudaMemcpyAsync(vals, vA, 4 * (size_t)n, cudaMemcpyDeviceToDevice, s));
   }
   return MGUSO_OK;
+}
+
+template <class K>
+static int sort_impl(Lbvh* b, K* keys, uint32_t* vals, uint32_t n, int key_bits, cudaStream_t s) {
+  if (n <= 1) return MGUSO_OK;
+  MG_TRY(b->rs_words.grow(rs_words(n, (key_bits + 7) / 8)));
+  MG_TRY(b->rs_tmpk.grow((size_t)n * sizeof(K)));
+  MG_TRY(b->rs_tmpv.grow(n));
+  return sort_run<K>(SortScratch{b->rs_words.p, b->rs_tmpk.p, b->rs_tmpv.p, b->err_sink ? b->err_sink : b->status.p},
+                     keys, vals, n, key_bits, 1, s);
 }
 
 int radix_sort_pairs(Lbvh* b, void* keys, uint32_t* vals, uint32_t n, int key_bits, cudaStream_t s) {
@@ -693,12 +739,11 @@ int lbvh_query_points(Lbvh* b, const float* pts, uint32_t np, float dhat, uint32
 constexpr uint32_t NOALLOC_MAX_PAIRS = 1u << 18;  // 262 144 pairs
 constexpr size_t NA_TMPK = 0;                                         // u64 keys, ping-pong
 constexpr size_t NA_TMPV = NA_TMPK + 8 * (size_t)NOALLOC_MAX_PAIRS;   // u32 payloads
-constexpr size_t NA_STATUS = NA_TMPV + 4 * (size_t)NOALLOC_MAX_PAIRS; // look-back flags
-constexpr size_t NA_HIST = NA_STATUS + 4 * 256 * (size_t)(NOALLOC_MAX_PAIRS / RS_TILE);
-constexpr size_t NA_OFS = NA_HIST + 4 * 8 * 256;
-constexpr size_t NA_MISC = NA_OFS + 4 * 8 * 256;  // [0] tile counter, [1] error word
-constexpr size_t NA_BYTES = NA_MISC + 256;         // 3.2 MiB per device
-static_assert(NOALLOC_MAX_PAIRS % RS_TILE == 0, "scratch holds whole tiles");
+constexpr size_t NA_WORDS = NA_TMPV + 4 * (size_t)NOALLOC_MAX_PAIRS;  // histograms, counters, look-back
+constexpr size_t NA_ERR =
+    NA_WORDS + (4 * 8 * (256 + 1 + 256 * (size_t)(NOALLOC_MAX_PAIRS / RS_TILE_S)) + 255) / 256 * 256;  // error word
+constexpr size_t NA_BYTES = NA_ERR + 256;  // 4.1 MiB per device
+static_assert(NOALLOC_MAX_PAIRS % RS_TILE_S == 0 && NOALLOC_MAX_PAIRS < RS_LARGE, "scratch holds whole small tiles");
 
 // Every device that loads the library holds this array until the process exits. Host code
 // must not pass the symbol itself to a kernel: its device address comes from
@@ -730,37 +775,11 @@ static int noalloc_scratch(unsigned char** out) {
 
 template <class K>
 static int noalloc_sort(unsigned char* sc, K* keys, uint32_t* vals, uint32_t n, int key_bits, cudaStream_t s) {
-  const int passes = (key_bits + 7) / 8;
-  const uint32_t ntiles = ceil_div(n, RS_TILE);
-  uint32_t* hist = (uint32_t*)(sc + NA_HIST);
-  uint32_t* ofs = (uint32_t*)(sc + NA_OFS);
-  uint32_t* status = (uint32_t*)(sc + NA_STATUS);
-  uint32_t* counter = (uint32_t*)(sc + NA_MISC);
-  uint32_t* err = counter + 1;
-  // the array keeps the previous call's contents: clear what the passes accumulate into
-  MG_CUDA(cudaMemsetAsync(hist, 0, 4 * 8 * 256, s));
+  uint32_t* err = (uint32_t*)(sc + NA_ERR);
+  // the array keeps the previous call's contents
   MG_CUDA(cudaMemsetAsync(err, 0, 4, s));
-  const int sms = device_sm_count();
-  k_rs_hist<K><<<std::min<uint32_t>(ceil_div(n, 256), sms * 8), 256, 0, s>>>(keys, n, passes, hist);
-  k_rs_scan<<<passes, 256, 0, s>>>(hist, ofs);
-  MG_CUDA(cudaGetLastError());
-  K* kA = keys;
-  uint32_t* vA = vals;
-  K* kB = (K*)(sc + NA_TMPK);
-  uint32_t* vB = (uint32_t*)(sc + NA_TMPV);
-  for (int p = 0; p < passes; ++p) {
-    MG_CUDA(cudaMemsetAsync(status, 0, 4 * (size_t)ntiles * 256, s));
-    MG_CUDA(cudaMemsetAsync(counter, 0, 4, s));
-    k_onesweep<K><<<ntiles, RS_THREADS, 0, s>>>(kA, vA, kB, vB, n, 8 * p, ofs + p * 256, status, counter, err,
-                                               nullptr);
-    MG_CUDA(cudaGetLastError());
-    std::swap(kA, kB);
-    std::swap(vA, vB);
-  }
-  if (kA != keys) {
-    MG_CUDA(cudaMemcpyAsync(keys, kA, sizeof(K) * (size_t)n, cudaMemcpyDeviceToDevice, s));
-    MG_CUDA(cudaMemcpyAsync(vals, vA, 4 * (size_t)n, cudaMemcpyDeviceToDevice, s));
-  }
+  MG_TRY(sort_run<K>(SortScratch{(uint32_t*)(sc + NA_WORDS), sc + NA_TMPK, (uint32_t*)(sc + NA_TMPV), err}, keys, vals,
+                     n, key_bits, 0, s));
   uint32_t h_err = 0;
   MG_CUDA(cudaMemcpyAsync(&h_err, err, 4, cudaMemcpyDeviceToHost, s));
   MG_CUDA(cudaStreamSynchronize(s));

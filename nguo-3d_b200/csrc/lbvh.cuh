@@ -29,7 +29,7 @@ struct Lbvh {
   DevBuf<uint32_t> status;
   uint32_t* err_sink = nullptr;     // when set, the sort's wait-timeout bit goes here instead of status
   // radix-sort scratch
-  DevBuf<uint32_t> rs_hist, rs_ofs, rs_status, rs_counter, rs_tmpv;
+  DevBuf<uint32_t> rs_words, rs_tmpv;
   DevBuf<unsigned char> rs_tmpk;
   // query scratch
   DevBuf<float4> qbox;
