@@ -1,4 +1,5 @@
 // extern "C" entry points of the LBVH broad phase and the radix sort.
+#include <cmath>
 #include <cstring>
 
 #include "lbvh.cuh"
@@ -12,7 +13,6 @@ int mguso_lbvh_create(mguso_ctx* ctx, mguso_lbvh** out) {
   MG_CUDA(cudaSetDevice(ctx->device));
   auto* b = new mguso_lbvh();
   b->b.ctx = ctx;
-  b->b.child_boxes = false;  // its point and box queries walk node and leaf boxes only
   *out = b;
   return MGUSO_OK;
 }
@@ -58,16 +58,25 @@ int mguso_lbvh_download(mguso_lbvh* b, uint64_t* keys, uint32_t* perm, uint32_t*
     }
   }
   if (perm && nt) MG_CUDA(cudaMemcpy(perm, L.perm.p, 4 * (size_t)nt, cudaMemcpyDeviceToHost));
-  if (nt > 1) {
-    if (left) MG_CUDA(cudaMemcpy(left, L.left.p, 4 * (size_t)(nt - 1), cudaMemcpyDeviceToHost));
-    if (right) MG_CUDA(cudaMemcpy(right, L.right.p, 4 * (size_t)(nt - 1), cudaMemcpyDeviceToHost));
-    if (node_boxes) {
-      std::vector<float4> nb(2 * (size_t)(nt - 1));
-      MG_CUDA(cudaMemcpy(nb.data(), L.node.p, sizeof(float4) * nb.size(), cudaMemcpyDeviceToHost));
-      for (uint32_t i = 0; i + 1 < nt; ++i) {
-        const float4 &lo = nb[2 * i], &hi = nb[2 * i + 1];
+  if (nt > 1 && (left || right || node_boxes)) {
+    // the children's indices and the node's box (their union) from its record
+    std::vector<float4> r(4 * (size_t)(nt - 1));
+    MG_CUDA(cudaMemcpy(r.data(), L.rec.p, sizeof(float4) * r.size(), cudaMemcpyDeviceToHost));
+    // as the refit's minima: a NaN gives way, -0 is below +0
+    auto least = [](float u, float v) { return u == v ? (std::signbit(u) ? u : v) : std::fmin(u, v); };
+    auto most = [](float u, float v) { return u == v ? (std::signbit(u) ? v : u) : std::fmax(u, v); };
+    for (uint32_t i = 0; i + 1 < nt; ++i) {
+      const float4 *a = &r[4 * (size_t)i], *b = a + 2;
+      if (left) std::memcpy(left + i, &a[0].w, 4);
+      if (right) std::memcpy(right + i, &b[0].w, 4);
+      if (node_boxes) {
         float* o = node_boxes + 6 * (size_t)i;
-        o[0] = lo.x; o[1] = lo.y; o[2] = lo.z; o[3] = hi.x; o[4] = hi.y; o[5] = hi.z;
+        o[0] = least(a[0].x, b[0].x);
+        o[1] = least(a[0].y, b[0].y);
+        o[2] = least(a[0].z, b[0].z);
+        o[3] = most(a[1].x, b[1].x);
+        o[4] = most(a[1].y, b[1].y);
+        o[5] = most(a[1].z, b[1].z);
       }
     }
   }

@@ -29,31 +29,10 @@ __device__ __forceinline__ bool excluded(const uint32_t* ex_ptr, const uint32_t*
   return false;
 }
 
-struct BvhView {
-  const uint32_t *left, *right, *prim;
-  const float4 *node, *leaf;
-  uint32_t n;
-  const float4 *dnode, *dleaf;  // displacement boxes of the same tree (CCD only)
-  const float4 *cbox, *dcbox;   // children's position and displacement boxes per inner node
-};
-
-static BvhView view(const Lbvh& b) {
-  return BvhView{b.left.p, b.right.p, b.perm.p, (const float4*)b.node.p, (const float4*)b.leaf.p, b.nt,
-                 (const float4*)b.dnode.p, (const float4*)b.dleaf.p, (const float4*)b.cbox.p,
-                 (const float4*)b.dcbox.p};
-}
-
-// One tree per instance over that instance's primitives (a query only meets its own
-// instance); base[k] turns a tree's local primitive index into the scene's.
-struct BvhSet {
-  BvhView t[PCG_MAX_INST];
-  uint32_t base[PCG_MAX_INST];
-};
-
 static BvhSet view_set(const std::vector<std::unique_ptr<Lbvh>>& b, const std::vector<uint32_t>& base) {
   BvhSet s{};
   for (size_t k = 0; k < b.size(); ++k) {
-    s.t[k] = view(*b[k]);
+    s.t[k] = lbvh_view(*b[k]);
     s.base[k] = base[k];
   }
   return s;
@@ -125,147 +104,6 @@ int build_bvhs(Scene& s, const float* x, bool refit) {
   }
   MG_TRY(aux_join(s));
   return rc;
-}
-
-// ---- warp walks -------------------------------------------------------------------------------
-// A warp takes `per` consecutive queries (up to 32) down their trees together: its queue holds
-// (query, node) pairs, each round takes up to 32 of them, newest first, one per lane, tests the
-// node's two children against the query and queues those entered; leaves go, as (query,
-// primitive) pairs, to a second queue, from which the whole warp takes 32 at a time through the
-// remaining filters and the narrow phase (distances, accd_toi). What bounds a walk is its chain
-// of dependent rounds: with a stack per lane, a warp ran as many rounds as its longest query
-// has nodes (some hundreds, about half of the lanes idle), while a shared queue keeps all
-// lanes on nodes of any query and needs little more than their number over 32, so that few
-// queries per warp (small scenes) spread over more warps. 64 x 64 sheet, before -> after: edge-edge
-// CCD 219 -> 87 us, vertex-triangle CCD 150 -> 30, stencils 140 -> 40 and 97 -> 22; one garment:
-// 160 -> 129, 176 -> 98, 145 -> 94 and 140 -> 49; six garments: 522 -> 421, 320 -> 243,
-// 408 -> 302 and 205 -> 122.
-// Results are order-free: stencils are sorted by their pair key afterwards, CCD results are
-// minima and sums, and the leaves reached do not depend on the order of the tests.
-constexpr int WQ_WARPS = 4;   // 128-thread blocks
-constexpr int WQ_QCAP = 96;   // < 32 left over + 2 leaves per lane and round
-// queued nodes per warp: a round adds at most 32; past FW_FULL one node is taken at a time, which
-// goes down depth first and adds at most one per level
-constexpr int FW_CAP = 1024, FW_FULL = FW_CAP - 128;
-
-template <class Q>
-struct WalkMem {  // shared memory of one warp
-  Q query[32];
-  uint32_t node[FW_CAP];
-  uint2 pair[WQ_QCAP];
-  uint8_t slot[FW_CAP];
-  uint8_t inst[32];
-};
-
-__device__ __forceinline__ void wq_push(uint2* q, int& n, bool has, uint2 e) {
-  const unsigned m = __ballot_sync(0xffffffffu, has);
-  if (has) q[n + __popc(m & ((1u << (threadIdx.x & 31)) - 1u))] = e;
-  n += __popc(m);
-}
-
-// Takes batches of up to 32 queued pairs while at least min_n are queued (n is warp-uniform).
-template <class F>
-__device__ __forceinline__ void wq_take(uint2* q, int& n, int min_n, F&& solve) {
-  const int lane = (int)(threadIdx.x & 31);
-  __syncwarp();
-  while (n >= min_n && n > 0) {
-    const int take = n < 32 ? n : 32;
-    const bool has = lane < take;
-    const uint2 e = has ? q[n - take + lane] : make_uint2(0u, 0u);
-    __syncwarp();
-    n -= take;
-    if (has) solve(e);
-  }
-}
-
-// Walks the trees of the warp's queries: lane l holds query l (valid or not) of instance k,
-// numbered first + l. keep(slot, primitive) says whether a leaf reached is to be solved.
-// Returns false when the node queue overflowed.
-template <class Q, class KEEP, class SOLVE>
-__device__ __forceinline__ bool warp_walk(WalkMem<Q>& m, const BvhSet& bs, uint32_t first, bool valid, uint32_t k,
-                                          const Q& mine, KEEP&& keep, SOLVE&& solve) {
-  const int lane = (int)(threadIdx.x & 31);
-  const unsigned below = (1u << lane) - 1u;
-  int n = 0, np = 0;
-  bool ok = true;
-  if (valid) {
-    m.query[lane] = mine;
-    m.inst[lane] = (uint8_t)k;
-  }
-  __syncwarp();
-  {
-    bool root = false, leaf = false;
-    uint32_t prim = 0;
-    if (valid) {
-      const BvhView& t = bs.t[k];
-      if (t.n == 1) {
-        leaf = mine.enter(__ldg(t.leaf), __ldg(t.leaf + 1), t.dleaf);
-        prim = bs.base[k] + __ldg(t.prim);
-      } else if (t.n > 1) {
-        root = mine.enter(__ldg(t.node), __ldg(t.node + 1), t.dnode);
-      }
-    }
-    const unsigned r = __ballot_sync(0xffffffffu, root);
-    if (root) {
-      const int at = __popc(r & below);
-      m.node[at] = 0;
-      m.slot[at] = (uint8_t)lane;
-    }
-    n = __popc(r);
-    if (leaf) leaf = keep((uint32_t)lane, prim);
-    wq_push(m.pair, np, leaf, make_uint2(first + lane, prim));
-  }
-  __syncwarp();
-  while (n > 0) {
-    const int take = n <= FW_FULL ? min(n, 32) : 1;
-    if (n + take > FW_CAP) {
-      ok = false;
-      break;
-    }
-    const bool has = lane < take;
-    uint32_t ch[2] = {0, 0}, slot = 0, base = 0;
-    const uint32_t* prims = nullptr;
-    bool in[2] = {false, false};
-    if (has) {
-      const uint32_t cur = m.node[n - take + lane];
-      slot = m.slot[n - take + lane];
-      const BvhView& t = bs.t[m.inst[slot]];
-      base = bs.base[m.inst[slot]];
-      prims = t.prim;
-      ch[0] = __ldg(t.left + cur);
-      ch[1] = __ldg(t.right + cur);
-      const float4* cb = t.cbox + 4 * (size_t)cur;
-      const float4* db = t.dcbox + 4 * (size_t)cur;
-      const float4 l0 = __ldg(cb), h0 = __ldg(cb + 1), l1 = __ldg(cb + 2), h1 = __ldg(cb + 3);
-      const Q& q = m.query[slot];
-      in[0] = q.enter(l0, h0, db);
-      in[1] = q.enter(l1, h1, db + 2);
-    }
-    n -= take;
-    __syncwarp();
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const bool inner = in[c] && !(ch[c] & LEAF_BIT);
-      const unsigned b = __ballot_sync(0xffffffffu, inner);
-      if (inner) {
-        const int at = n + __popc(b & below);
-        m.node[at] = ch[c];
-        m.slot[at] = (uint8_t)slot;
-      }
-      n += __popc(b);
-      bool leaf = in[c] && (ch[c] & LEAF_BIT);
-      uint32_t prim = 0;
-      if (leaf) {
-        prim = base + __ldg(prims + (ch[c] & ~LEAF_BIT));
-        leaf = keep(slot, prim);
-      }
-      wq_push(m.pair, np, leaf, make_uint2(first + slot, prim));
-    }
-    wq_take(m.pair, np, 32, solve);
-    __syncwarp();
-  }
-  wq_take(m.pair, np, 1, solve);
-  return ok;
 }
 
 // Queries per warp: as many as leave every SM some warps (a walk's rounds are latency-bound), up
