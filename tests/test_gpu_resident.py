@@ -100,3 +100,27 @@ def test_staged_fp16_domains_match_the_fused_kernels(ctx):
     disp = np.abs(out[0][0] - sc["positions"]).max()
     assert np.abs(out[0][0] - out[1][0]).max() <= 1e-3 * disp
     assert abs(out[0][1]["max_cg_iters"] - out[1][1]["max_cg_iters"]) <= 2
+
+
+@pytest.mark.parametrize("precond", ["schwarz", "block"])
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+def test_non_finite_values_end_fp64_solves_as_fp32_ones(ctx, precond, bad):
+    """FP64 sums take their FP32 operands' bits, which have no infinity or NaN: such rows go another
+    way and the solve has to end where the FP32 one (plain conversions) does."""
+    nb, rp, col, val = scenes.grid_bsr(12, 4)
+    val = val.copy()
+    v = 77  # an off-diagonal block, so that the diagonal stays what the preconditioner expects
+    k = next(k for k in range(rp[v], rp[v + 1]) if col[k] != v)
+    val[k, 1, 2] = bad
+    a = CsrMatrix(*scenes.bsr_to_csr(nb, rp, col, val))
+    b = np.random.default_rng(2).standard_normal(3 * nb).astype(np.float32)
+    ends = []
+    for precision in ("fp32", "mixed"):
+        s = CudaLinearSolver(ctx, precond=precond, domain=32, precision=precision)
+        try:
+            x = s.solve(a, b, 1e-6, 500)
+            ends.append((s.last_stats().status, s.last_stats().iters, np.isfinite(x).all()))
+        except Exception as e:
+            ends.append(type(e).__name__)
+        s.close()
+    assert ends[0] == ends[1]
