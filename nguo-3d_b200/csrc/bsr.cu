@@ -62,6 +62,25 @@ int bsr_build_host_from_csr(const mguso_csr* a, uint32_t& nb, std::vector<uint32
   return MGUSO_OK;
 }
 
+// Values of an unchanged pattern from the scalar CSR's, on the device: each value knows its entry,
+// so writes are whole lines and nothing is zeroed first. (Scattered on the host into a zeroed
+// copy of the blocks, which then had to be uploaded: 2.5 of 8.1 ms for 229 000 blocks.)
+__global__ void k_gather_csr(const float* __restrict__ values, const uint32_t* __restrict__ src, uint32_t n,
+                             float* __restrict__ val) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t k = src[i];
+  val[i] = 0.0f + (k == CSR_NONE ? 0.0f : __ldg(values + k));  // a sum from 0, as on a first solve (-0 to 0)
+}
+
+int bsr_gather_csr(mguso_bsr* a, const float* values, const uint32_t* src, cudaStream_t s) {
+  const uint32_t n = 9 * a->nnzb;
+  if (n == 0) return MGUSO_OK;
+  k_gather_csr<<<ceil_div(n, 256), 256, 0, s>>>(values, src, n, a->val.p);
+  MG_CUDA(cudaGetLastError());
+  return MGUSO_OK;
+}
+
 int bsr_upload(mguso_bsr* m, uint32_t nb, const std::vector<uint32_t>& row_ptr, const std::vector<uint32_t>& col,
                const float* val_host) {
   cudaStream_t s = m->ctx->stream;

@@ -264,18 +264,32 @@ int mguso_linear_solve(mguso_linear_solver* s, const mguso_csr* a, const float* 
     std::vector<uint32_t> rp, cl;
     std::vector<float> val;
     MG_TRY(bsr_build_host_from_csr(a, nb, rp, cl, val));
+    s->csr_row_ptr.clear();  // no pattern, should what follows fail
     s->bsr = std::make_unique<mguso_bsr>();
     s->bsr->ctx = s->ctx;
     MG_TRY(bsr_upload(s->bsr.get(), nb, rp, cl, val.data()));
-    // scalar entry -> BSR value slot, so a re-solve on the same pattern scatters values only
+    // where a re-solve on the same pattern finds its values; an entry that is there twice is
+    // summed on the host, in the entries' order
+    std::vector<uint32_t> src((size_t)9 * s->bsr->nnzb, CSR_NONE);
+    bool twice = false;
     s->map_val.resize(nnz);
     for (uint32_t row = 0; row < a->n; ++row) {
-      uint32_t v = row / 3;
+      uint32_t v = row / 3, j = rp[v];
       for (uint32_t k = a->row_ptr[row]; k < a->row_ptr[row + 1]; ++k) {
         uint32_t cb = a->col_idx[k] / 3;
-        uint32_t j = (uint32_t)(std::lower_bound(cl.begin() + rp[v], cl.begin() + rp[v + 1], cb) - cl.begin());
-        s->map_val[k] = 9 * j + 3 * (row % 3) + a->col_idx[k] % 3;
+        if (cl[j] != cb && !(++j < rp[v + 1] && cl[j] == cb))  // columns in order: this block or the next
+          j = (uint32_t)(std::lower_bound(cl.begin() + rp[v], cl.begin() + rp[v + 1], cb) - cl.begin());
+        const uint32_t at = 9 * j + 3 * (row % 3) + a->col_idx[k] % 3;
+        twice = twice || src[at] != CSR_NONE;
+        src[at] = k;
+        s->map_val[k] = at;
       }
+    }
+    if (twice) {
+      s->src_val.release();
+    } else {
+      s->map_val = {};
+      MG_TRY(s->src_val.upload(src.data(), src.size(), st));
     }
     s->csr_row_ptr.assign(a->row_ptr, a->row_ptr + a->n + 1);
     s->csr_col.assign(a->col_idx, a->col_idx + nnz);
@@ -290,6 +304,10 @@ int mguso_linear_solve(mguso_linear_solver* s, const mguso_csr* a, const float* 
       s->schwarz->pack_singles = s->levels != 2;  // two levels: every domain a coarse node, as the reference
       MG_TRY(schwarz_build(s->schwarz.get()));
     }
+  } else if (s->src_val.p) {
+    MG_TRY(s->csr_val.reserve(nnz));
+    MG_CUDA(cudaMemcpyAsync(s->csr_val.p, a->values, 4 * (size_t)nnz, cudaMemcpyHostToDevice, st));
+    MG_TRY(bsr_gather_csr(s->bsr.get(), s->csr_val.p, s->src_val.p, st));
   } else {
     s->h_val.assign((size_t)9 * s->bsr->nnzb, 0.0f);
     for (uint32_t k = 0; k < nnz; ++k) s->h_val[s->map_val[k]] += a->values[k];

@@ -276,11 +276,17 @@ struct mguso_linear_solver {
   mg::DevBuf<mg::FusedInst> rs_inst;
   mg::PinnedBuf<mg::FusedInst> rs_out;
   uint64_t generation = 0;         // bumped whenever the pattern is rebuilt
-  std::vector<uint32_t> map_val;   // scalar CSR entry -> BSR value slot
+  // a re-solve's values: each BSR value's scalar CSR entry (CSR_NONE: a zero of its block), or, where
+  // a pattern names an entry twice, each entry's BSR value
+  mg::DevBuf<uint32_t> src_val;
+  mg::DevBuf<float> csr_val;
+  std::vector<uint32_t> map_val;
   std::vector<float> h_val;
 };
 
 namespace mg {
 int pcg_solve(mguso_linear_solver* s, float tol, uint32_t max_iter, mguso_lin_stats* st);
 int blockjacobi_factor(mguso_bsr* a, float* inv, cudaStream_t s);
+constexpr uint32_t CSR_NONE = 0xffffffffu;
+int bsr_gather_csr(mguso_bsr* a, const float* values, const uint32_t* src, cudaStream_t s);
 }  // namespace mg
