@@ -111,8 +111,7 @@ struct mguso_schwarz {
   std::vector<uint32_t> h_cdom_start, h_cdom_nodes;
   mg::DevBuf<uint32_t> cdom_start;  // ncdom + 1
   mg::DevBuf<uint32_t> cdom_nodes;  // ndom: coarse nodes (level-0 domains) by coarse domain
-  mg::DevBuf<uint32_t> cdom_of;     // ndom: coarse domain of each coarse node
-  mg::DevBuf<uint32_t> cloc;        // ndom: local index of a coarse node in its coarse domain
+  mg::DevBuf<uint2> cplace;         // nb: the vertex's coarse domain and its coarse node's place in it
   mg::DevBuf<uint32_t> dom_sorted;  // nb: each level-0 domain's vertices in ascending order
   mg::DevBuf<uint64_t> cfac_off;    // ncdom + 1
   mg::DevBuf<float> cfac;           // W1 tiles

@@ -198,8 +198,9 @@ int schwarz_build_coarse(mguso_schwarz* s) {
   cudaStream_t st = a->ctx->stream;
   MG_TRY(s->cdom_start.upload(s->h_cdom_start.data(), s->h_cdom_start.size(), st));
   MG_TRY(s->cdom_nodes.upload(s->h_cdom_nodes.data(), std::max<size_t>(s->h_cdom_nodes.size(), 1), st));
-  MG_TRY(s->cdom_of.upload(cdom_of.data(), std::max<size_t>(nd, 1), st));
-  MG_TRY(s->cloc.upload(cloc.data(), std::max<size_t>(nd, 1), st));
+  std::vector<uint2> place(std::max<uint32_t>(a->nb, 1));
+  for (uint32_t v = 0; v < a->nb; ++v) place[v] = make_uint2(cdom_of[s->h_dom_of[v]], cloc[s->h_dom_of[v]]);
+  MG_TRY(s->cplace.upload(place.data(), place.size(), st));
   MG_TRY(s->dom_sorted.upload(sorted.data(), std::max<size_t>(sorted.size(), 1), st));
   MG_TRY(s->cfac_off.upload(off.data(), off.size(), st));
   MG_TRY(s->cfac.reserve(std::max<uint64_t>(off[s->ncdom], 4)));
@@ -300,26 +301,34 @@ __global__ void __launch_bounds__(32 * WARPS) k_schwarz_apply(
   if (with_dot == 1) grid_dot_commit<Acc>(dot, acc);
 }
 
-// Coarse level of the two-level apply, one warp per coarse domain: restriction
+// Coarse level of the two-level apply, one CTA per coarse domain: restriction
 // rc = sum of r over each coarse node's vertices (linsolve.rs:648-655), the domain's
-// z1 = W1^T (W1 rc) from its FP32 tiles, written as the coarse correction ec.
-__global__ void __launch_bounds__(32) k_coarse_apply(
+// z1 = W1^T (W1 rc) from its FP32 tiles, written as the coarse correction ec. A few hundred coarse
+// domains do not fill the chip, so the chain in one of them is the time: a warp per coarse node
+// (with one warp for all, its 16 to 32 nodes' gathers ran one after another) and a warp per
+// tile in both products, whose partial sums are added in storage order. 200 x 200 grid,
+// 16-vertex domains: 20.6 -> 6.2 us.
+constexpr int CA_WARPS = 8;
+
+__global__ void __launch_bounds__(32 * CA_WARPS) k_coarse_apply(
     const uint32_t* __restrict__ cdom_start, const uint32_t* __restrict__ cdom_nodes,
     const uint32_t* __restrict__ dom_start, const uint32_t* __restrict__ dom_verts,
     const uint64_t* __restrict__ cfac_off, const float* __restrict__ cfac, const float* __restrict__ r,
     float* __restrict__ ec, uint32_t ncdom, const PcgScalars* done) {
   __shared__ __align__(16) float buf[6 * TILE_FLOATS];
   __shared__ float rd[96];
-  __shared__ double yd[96];
+  __shared__ double yd[96], part[6][32];
   if (done && done->done) return;
-  const int lane = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   for (uint32_t d1 = blockIdx.x; d1 < ncdom; d1 += gridDim.x) {
     const uint32_t n0 = cdom_start[d1], mn = cdom_start[d1 + 1] - n0;
-    const int m = 3 * (int)mn;
+    const int m = 3 * (int)mn, T = (m + 31) >> 5;
     const uint64_t off = cfac_off[d1];
-    const int nfl = (int)(cfac_off[d1 + 1] - off);
-    for (int e = lane; e < nfl; e += 32) buf[e] = cfac[off + e];
-    for (uint32_t a = 0; a < mn; ++a) {
+    const int n4 = (int)(cfac_off[d1 + 1] - off) / 4;  // whole tiles
+    for (int e = tid; e < n4; e += 32 * CA_WARPS)
+      reinterpret_cast<float4*>(buf)[e] = __ldg(reinterpret_cast<const float4*>(cfac + off) + e);
+#pragma unroll 4
+    for (uint32_t a = w; a < mn; a += CA_WARPS) {
       const uint32_t g = cdom_nodes[n0 + a];
       double s0 = 0, s1 = 0, s2 = 0;
       for (uint32_t p = dom_start[g] + lane; p < dom_start[g + 1]; p += 32) {
@@ -337,22 +346,38 @@ __global__ void __launch_bounds__(32) k_coarse_apply(
         rd[3 * a + 2] = (float)s2;
       }
     }
-    for (int i = m + lane; i < 96; i += 32) rd[i] = 0.f;
-    __syncwarp();
-    double zz[3];
-    const int T = (m + 31) >> 5;
-    if (T == 3)
-      tiles_apply<3, double, float>(buf, rd, yd, zz, lane);
-    else if (T == 2)
-      tiles_apply<2, double, float>(buf, rd, yd, zz, lane);
-    else
-      tiles_apply<1, double, float>(buf, rd, yd, zz, lane);
-#pragma unroll
-    for (int J = 0; J < 3; ++J) {
-      const int i = 32 * J + lane;
-      if (i < m) ec[3 * cdom_nodes[n0 + i / 3] + i % 3] = (float)zz[J];
+    for (int i = m + tid; i < 96; i += 32 * CA_WARPS) rd[i] = 0.f;
+    __syncthreads();
+    const int I = w >= 3 ? 2 : (w >= 1 ? 1 : 0), J = w - I * (I + 1) / 2;  // this warp's tile
+    const bool mine = w < T * (T + 1) / 2;
+    const float* t = buf + w * TILE_FLOATS;
+    if (mine) {
+      double y = 0;
+#pragma unroll 8
+      for (int c = 0; c < 32; ++c) y += (double)tile_ld(t, tile_off<float>(lane, c)) * (double)rd[32 * J + c];
+      part[w][lane] = y;
     }
-    __syncwarp();
+    __syncthreads();
+    if (w < T) {
+      double y = part[w * (w + 1) / 2][lane];
+      for (int k = 1; k <= w; ++k) y += part[w * (w + 1) / 2 + k][lane];
+      yd[32 * w + lane] = y;
+    }
+    __syncthreads();
+    if (mine) {
+      double z = 0;
+#pragma unroll 8
+      for (int k = 0; k < 32; ++k) z += (double)tile_ld(t, tile_off<float>(k, lane)) * yd[32 * I + k];
+      part[w][lane] = z;
+    }
+    __syncthreads();
+    const int i = 32 * w + lane;
+    if (w < T && i < m) {
+      double z = part[w * (w + 1) / 2 + w][lane];
+      for (int k = w + 1; k < T; ++k) z += part[k * (k + 1) / 2 + w][lane];
+      ec[3 * cdom_nodes[n0 + i / 3] + i % 3] = (float)z;
+    }
+    __syncthreads();
   }
 }
 
@@ -427,8 +452,8 @@ int schwarz_apply(mguso_schwarz* s, const float* r, float* z, cudaStream_t st, c
   if (grid == 0) return MGUSO_OK;
   MG_CUDA(cudaLaunchKernel(fn, dim3(grid), dim3(32 * APPLY_WARPS), args, smem, st));
   if (s->levels != 2 || s->ncdom == 0) return MGUSO_OK;
-  const uint32_t cgrid = std::min<uint32_t>(s->ncdom, 16u * (uint32_t)s->a->ctx->sm_count);
-  k_coarse_apply<<<cgrid, 32, 0, st>>>(s->cdom_start.p, s->cdom_nodes.p, s->dom_start.p, s->dom_verts.p,
+  const uint32_t cgrid = std::min<uint32_t>(s->ncdom, 8u * (uint32_t)s->a->ctx->sm_count);
+  k_coarse_apply<<<cgrid, 32 * CA_WARPS, 0, st>>>(s->cdom_start.p, s->cdom_nodes.p, s->dom_start.p, s->dom_verts.p,
                                        s->cfac_off.p, s->cfac.p, r, s->ec.p, s->ncdom, dot ? dot->sc : nullptr);
   const uint32_t nb = s->a->nb;
   const uint32_t pgrid = std::max<uint32_t>(1, std::min<uint32_t>(ceil_div(nb, 256), 8u * (uint32_t)s->a->ctx->sm_count));
