@@ -215,8 +215,10 @@ struct RsRun {
 };
 
 struct RsWork {
-  void* fn = nullptr;  // the kernel variant `smem` was found for
-  uint32_t smem = 0;   // its dynamic shared memory; 0: it cannot be resident on this device
+  // per team size: the kernel that `smem` was found for and its dynamic shared memory (0: it cannot
+  // be resident on this device)
+  void* fn[2] = {nullptr, nullptr};
+  uint32_t smem[2] = {0, 0};
   DevBuf<float4> rec;
   DevBuf<float> jscr;
   DevBuf<uint4> sums;

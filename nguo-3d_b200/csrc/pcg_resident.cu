@@ -6,8 +6,8 @@
 // What bounds a drape's PCG iteration is not its bytes but its chain of dependent steps: as two
 // kernels per iteration it took 17 us for a 4 096-vertex sheet and 25 us for a 31 000-vertex
 // garment, most of it launches, dependent loads from L2 and the last-CTA reductions (45 us for
-// six garments, 137 MB an iteration). So here one CTA stays on each SM for the whole solve: 6.9,
-// 10 and 34 us an iteration. What is left: two exchanges of 2.5 to 3 thousand cycles (1.3 thousand
+// six garments, 137 MB an iteration). So here one CTA stays on each SM for the whole solve: 6.1,
+// 9.5 and 33 us an iteration. What is left: two exchanges of 2.5 to 3 thousand cycles (1.3 thousand
 // is what a store takes to be seen by another SM and read back), 1 to 1.5 thousand for the halo,
 // and one warp's instruction chain in each phase.
 //  - a CTA owns a run of Schwarz domains (block Jacobi: runs of 32 vertices), the domains'
@@ -29,8 +29,8 @@
 //    epoch too, so what is read too early is seen to be and read again: no fence. Instances
 //    of a batch never wait for another.
 // Three warps (a team) take one domain at a time: for the rows each warp takes every third
-// block of a row, for the preconditioner every third tile (six warps were no faster: 64
-// registers a thread spill).
+// block of a row, for the preconditioner every third tile. Where a CTA has three domains or
+// fewer, six warps do (36 warps in six such teams were no faster: 64 registers a thread spill).
 //
 // The CTAs are resident together (cooperative launch). Every poll is bounded: a CTA that gives
 // up sets its instance's status and leaves, and the others follow. Dot products are summed in a
@@ -45,19 +45,15 @@
 
 namespace mg {
 
-constexpr int RS_TEAMS = 6;
-constexpr int RS_TW = 3;              // warps of a team
-constexpr int RS_TEAM = 32 * RS_TW;
-constexpr int RS_THREADS = RS_TEAM * RS_TEAMS;
-constexpr int RS_WARPS = RS_THREADS / 32;
+constexpr int RS_WARPS = 18;          // six teams of three warps, or three of six
+constexpr int RS_THREADS = 32 * RS_WARPS;
 constexpr int RS_MAX_DOM = 64;       // domains (of <= 32 vertices) per CTA
 constexpr uint32_t RS_HASH = 4096;   // halo hash table entries
 constexpr uint32_t RS_PROBES = 64;   // a column not placed within these is read from global
 constexpr uint32_t RS_MAX_HALO = 1536;
 constexpr uint32_t RS_HASH_BYTES = RS_HASH * 6;
-constexpr uint32_t RS_TEAM_BYTES = 2688;  // per-team scratch
+constexpr uint32_t RS_SCRATCH = 16128;    // the teams' scratch
 constexpr uint32_t RS_CHUNK = 12288;      // a staging buffer (an FP16 domain's tiles); two per team
-constexpr uint32_t RS_CHUNK_SLOTS = 9;    // whole slots of packed rows per chunk
 constexpr uint32_t RS_EMPTY = 0xffffffffu;
 constexpr uint32_t RS_WIDE = 8;  // rows that make a slot worth padding to 32
 constexpr uint32_t RS_ALWAYS = 0xffffffffu;  // epoch of a record that holds for the whole solve
@@ -108,8 +104,9 @@ __device__ __forceinline__ double rs_widen(float v, double) {
 __device__ __forceinline__ float rs_lift(float v) { return v; }
 __device__ __forceinline__ double rs_lift(double v) { return v * 0x1p448; }
 
-__device__ __forceinline__ void team_sync(int team) {
-  asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "n"(RS_TEAM) : "memory");
+template <int THREADS>
+__device__ __forceinline__ void team_sync_of(int team) {
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "n"(THREADS) : "memory");
 }
 // 16 bytes as one access: a record or a published sum and its epoch arrive together
 __device__ __forceinline__ uint4 ld_rlx(const void* p) {
@@ -302,10 +299,14 @@ struct StageNext {
   uint32_t part, tiles, issued;
 };
 
-template <int PRE, class Acc, class TS>
+template <int PRE, class Acc, class TS, int TW>
 __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_constant__ RsArgs a) {
   constexpr bool SCH = PRE == MGUSO_PRECOND_SCHWARZ;
   using AA = typename std::conditional<sizeof(TS) == 2, float, Acc>::type;
+  constexpr int TEAMS = RS_WARPS / TW, TEAM = 32 * TW;
+  constexpr uint32_t TEAM_BYTES = RS_SCRATCH / TEAMS;  // per-team scratch
+  constexpr uint32_t CHUNK_SLOTS = TW == 3 ? 9 : 6;    // whole slots of packed rows per chunk: a multiple of TW
+  auto team_sync = [](int t) { team_sync_of<TEAM>(t); };
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ uint32_t s_dpos[RS_MAX_DOM + 1];  // first own vertex of each domain
   __shared__ uint32_t s_bytes[RS_MAX_DOM];  // of the packed rows
@@ -314,8 +315,8 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
   __shared__ float s_scale[RS_MAX_DOM];
   __shared__ uint8_t s_jmode[RS_MAX_DOM];  // 0 shared memory, 1 staged from global scratch, 2 the BSR itself
   __shared__ uint8_t s_far[RS_MAX_DOM];
-  __shared__ StageNext s_sg[RS_TEAMS];
-  __shared__ __align__(8) uint64_t s_bar[2 * RS_TEAMS];
+  __shared__ StageNext s_sg[TEAMS];
+  __shared__ __align__(8) uint64_t s_bar[2 * TEAMS];
   __shared__ uint16_t s_len[RS_MAX_DOM * 32];
   __shared__ uint8_t s_row[RS_MAX_DOM * 32];
   __shared__ Acc s_red[2][RS_WARPS];
@@ -325,7 +326,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
   __shared__ uint32_t s_nh, s_nlive, s_done, s_abort;
   __shared__ uint32_t s_stage;  // first byte of the staging buffers (0: none)
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int team = wid / RS_TW, q = wid - RS_TW * team, ti = 32 * q + lane;
+  const int team = wid / TW, q = wid - TW * team, ti = 32 * q + lane;
   const RsSystem& S = a.sys;
 
   uint32_t ii = 0;
@@ -355,8 +356,8 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
     s_nh = 0;
     s_done = 0;
     s_abort = 0;
-    for (int t = 0; t < 2 * RS_TEAMS; ++t) mbar_init(&s_bar[t], 1);
-    for (int t = 0; t < RS_TEAMS; ++t) s_sg[t] = StageNext{t, 0u, SCH ? 1u : 0u, 0u};
+    for (int t = 0; t < 2 * TEAMS; ++t) mbar_init(&s_bar[t], 1);
+    for (int t = 0; t < TEAMS; ++t) s_sg[t] = StageNext{t, 0u, SCH ? 1u : 0u, 0u};
     fence_mbar_init();
     s_alpha = 0.f;
     s_beta = 0.f;
@@ -417,7 +418,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
   // only the others ("live") are iterated; listed in order by one warp
   __syncthreads();
   const uint32_t H = min(s_nh, RS_MAX_HALO);
-  float4* xs = reinterpret_cast<float4*>(smem + RS_TEAMS * RS_TEAM_BYTES);  // p of own vertices, then of the halo
+  float4* xs = reinterpret_cast<float4*>(smem + TEAMS * TEAM_BYTES);  // p of own vertices, then of the halo
   float* rv = reinterpret_cast<float*>(xs + own + H);
   float* az = rv + 3 * own;  // Ap after the rows, z after the preconditioner
   float* xv = az + 3 * own;  // the solution
@@ -461,8 +462,8 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
       all += SCH ? (S.fac_off[d0 + di + 1] - S.fac_off[d0 + di]) * sizeof(TS) : (36u * (s_dpos[di + 1] - s_dpos[di]) + 15u) & ~15u;
     }
     uint32_t top = a.smem_bytes;
-    if (all > a.smem_bytes && cur + 2 * RS_TEAMS * RS_CHUNK <= a.smem_bytes)
-      top -= 2 * RS_TEAMS * RS_CHUNK;
+    if (all > a.smem_bytes && cur + 2 * TEAMS * RS_CHUNK <= a.smem_bytes)
+      top -= 2 * TEAMS * RS_CHUNK;
     s_stage = top < a.smem_bytes ? top : 0u;
     const uint32_t lim = min(top, a.smem_bytes - RS_HASH_BYTES);
     for (int di = 0; di < nD; ++di) {
@@ -487,8 +488,8 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
   auto jbase = [&](int di) -> float* {
     return s_jmode[di] ? a.jscr + 4 * (size_t)s_jofs[di] : reinterpret_cast<float*>(smem + s_jofs[di]);
   };
-  for (int u = wid; u < RS_TW * nD; u += RS_WARPS) {
-    const int di = u / RS_TW, uq = u - RS_TW * di;
+  for (int u = wid; u < TW * nD; u += RS_WARPS) {
+    const int di = u / TW, uq = u - TW * di;
     if (s_jmode[di] == 2) continue;  // uniform
     const uint32_t len = s_len[32 * di + lane], maxlen = s_len[32 * di], wide = s_wide[di], nt = s_tail[di];
     const uint32_t row = s_row[32 * di + lane];
@@ -522,7 +523,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
       far = true;
       return 0;
     };
-    for (uint32_t sj = uq; sj < wide; sj += RS_TW) {
+    for (uint32_t sj = uq; sj < wide; sj += TW) {
       float m[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
       uint32_t code = 0;
       if (sj < len) code = fetch(sj, m);
@@ -534,7 +535,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
     uint32_t o = 0;
     for (uint32_t sj = wide; sj < maxlen; ++sj) {
       const uint32_t cnt = __popc(__ballot_sync(0xffffffffu, len > sj));
-      if (sj % RS_TW == (uint32_t)uq && (uint32_t)lane < cnt) {
+      if (sj % TW == (uint32_t)uq && (uint32_t)lane < cnt) {
         float m[9];
         const uint32_t code = fetch(sj, m);
 #pragma unroll
@@ -564,13 +565,13 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
     }
   }
   __syncthreads();
-  for (int di = team; di < nD; di += RS_TEAMS) {
+  for (int di = team; di < nD; di += TEAMS) {
     if (SCH && sizeof(AA) > sizeof(TS) && sizeof(TS) == 4) {
       // a tile that rs_widen cannot take: its domain's z is NaN, as its product would be
       const uint32_t n = (uint32_t)(S.fac_off[d0 + di + 1] - S.fac_off[d0 + di]);
       const float* src = (const float*)S.fac + S.fac_off[d0 + di];
       bool bad = false;
-      for (uint32_t i = ti; i < n; i += RS_TEAM) bad = bad || !rs_finite(__ldg(src + i));
+      for (uint32_t i = ti; i < n; i += TEAM) bad = bad || !rs_finite(__ldg(src + i));
       if (bad) s_scale[di] = __uint_as_float(0x7fffffffu);
     }
     if (s_tofs[di] == RS_EMPTY) continue;
@@ -578,16 +579,16 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
       const uint32_t n16 = (uint32_t)((S.fac_off[d0 + di + 1] - S.fac_off[d0 + di]) * sizeof(TS)) / 16;
       const uint4* src = reinterpret_cast<const uint4*>((const TS*)S.fac + S.fac_off[d0 + di]);
       uint4* dst = reinterpret_cast<uint4*>(smem + s_tofs[di]);
-      for (uint32_t i = ti; i < n16; i += RS_TEAM) dst[i] = __ldg(src + i);
+      for (uint32_t i = ti; i < n16; i += TEAM) dst[i] = __ldg(src + i);
     } else {
       const uint32_t nf = 9 * (s_dpos[di + 1] - s_dpos[di]);
       const float* src = S.bjinv + 9 * (size_t)(P0 + s_dpos[di]);
       float* dst = reinterpret_cast<float*>(smem + s_tofs[di]);
-      for (uint32_t i = ti; i < nf; i += RS_TEAM) dst[i] = __ldg(src + i);
+      for (uint32_t i = ti; i < nf; i += TEAM) dst[i] = __ldg(src + i);
     }
   }
 
-  unsigned char* tscr = smem + team * RS_TEAM_BYTES;
+  unsigned char* tscr = smem + team * TEAM_BYTES;
   uint4* sums = a.sums + I.cta0;
   uint32_t* count = a.count + 32 * ii;
   uint32_t target = 0;  // the counter once all have published
@@ -603,15 +604,15 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
   // rows' chunks: runs of whole slots, the blocks past them in the last run's chunk if they fit
   auto row_chunks = [&](int di, bool& joined) -> uint32_t {
     const uint32_t wide = s_wide[di], tail = s_bytes[di] - 1280u * wide;
-    const uint32_t nw = (wide + RS_CHUNK_SLOTS - 1) / RS_CHUNK_SLOTS;
-    joined = nw > 0 && 1280u * (wide - (nw - 1) * RS_CHUNK_SLOTS) + tail <= RS_CHUNK;
+    const uint32_t nw = (wide + CHUNK_SLOTS - 1) / CHUNK_SLOTS;
+    joined = nw > 0 && 1280u * (wide - (nw - 1) * CHUNK_SLOTS) + tail <= RS_CHUNK;
     return nw + ((tail && !joined) ? 1u : 0u);
   };
   auto stage_issue = [&]() {  // the team's first thread
     if (ti != 0 || !s_stage) return;
     StageNext n = s_sg[team];
     for (int turn = 0; turn < 3; ++turn) {
-      for (; n.di < nD; n.di += RS_TEAMS) {
+      for (; n.di < nD; n.di += TEAMS) {
         if (!(n.tiles ? staged_tile(n.di) : staged_row(n.di))) continue;
         const unsigned char* src;
         uint32_t bytes;
@@ -623,10 +624,10 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
         } else {
           bool joined;
           const uint32_t nc = row_chunks(n.di, joined);
-          const uint32_t start = min(1280u * RS_CHUNK_SLOTS * n.part, 1280u * s_wide[n.di]);
+          const uint32_t start = min(1280u * CHUNK_SLOTS * n.part, 1280u * s_wide[n.di]);
           last = n.part + 1 == nc;
           src = reinterpret_cast<const unsigned char*>(a.jscr + 4 * (size_t)s_jofs[n.di]) + start;
-          bytes = last ? s_bytes[n.di] - start : min(1280u * RS_CHUNK_SLOTS, 1280u * s_wide[n.di] - start);
+          bytes = last ? s_bytes[n.di] - start : min(1280u * CHUNK_SLOTS, 1280u * s_wide[n.di] - start);
         }
         uint64_t* bar = &s_bar[2 * team + (n.issued & 1u)];
         mbar_arrive_expect_tx(bar, bytes);
@@ -634,7 +635,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
         ++n.issued;
         ++n.part;
         if (last) {
-          n.di += RS_TEAMS;
+          n.di += TEAMS;
           n.part = 0;
         }
         s_sg[team] = n;
@@ -797,19 +798,19 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
     for (uint32_t e = tid; e < 3 * nlive; e += RS_THREADS) lp[e] = fmaf(be, lp[e], lz[e]);
     __syncthreads();
     Acc acc = 0;
-    Acc* part = reinterpret_cast<Acc*>(tscr);  // [RS_TW][96]
-    for (int di = team; di < nD; di += RS_TEAMS) {
+    Acc* part = reinterpret_cast<Acc*>(tscr);  // [TW][96]
+    for (int di = team; di < nD; di += TEAMS) {
       const uint32_t row = s_row[32 * di + lane], dp = s_dpos[di], dn = s_dpos[di + 1], wide = s_wide[di];
       const int mode = s_jmode[di];
       Acc y0 = 0, y1 = 0, y2 = 0;
       if (mode == 2) {
-        if (dp + row < dn) bsr_row(vert(P0 + dp + row), q, RS_TW, epoch, be, y0, y1, y2);
+        if (dp + row < dn) bsr_row(vert(P0 + dp + row), q, TW, epoch, be, y0, y1, y2);
       } else {
         const unsigned char* xb = reinterpret_cast<const unsigned char*>(xs);
         // whole slots q, q + 3, .. below `n` of the run at `jv`
         auto whole = [&](const unsigned char* jv, uint32_t n) {
 #pragma unroll 2
-          for (uint32_t sj = q; sj < n; sj += RS_TW) {
+          for (uint32_t sj = q; sj < n; sj += TW) {
             const float4* s4 = reinterpret_cast<const float4*>(jv) + 80 * sj + lane;
             const float4 ma = s4[0], mb = s4[32];
             const float2 mc = *reinterpret_cast<const float2*>(jv + 1280 * sj + 1024 + 8 * lane);
@@ -832,7 +833,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
           uint32_t o = 0;
           for (uint32_t sj = wide; sj < maxlen; ++sj) {
             const uint32_t cnt = __popc(__ballot_sync(0xffffffffu, len > sj));
-            if (sj % RS_TW == (uint32_t)q && (uint32_t)lane < cnt) {
+            if (sj % TW == (uint32_t)q && (uint32_t)lane < cnt) {
               const float* m = tv + 9 * o + lane;
               const float4 x = *reinterpret_cast<const float4*>(
                   xb + reinterpret_cast<const uint32_t*>(tv + 9 * (size_t)nt)[o + lane]);
@@ -859,7 +860,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
           const uint32_t n = row_chunks(di, joined);
           for (uint32_t c = 0; c < n; ++c) {
             const unsigned char* b = stage_wait();
-            const uint32_t first = min(RS_CHUNK_SLOTS * c, wide), here = min(RS_CHUNK_SLOTS, wide - first);
+            const uint32_t first = min(CHUNK_SLOTS * c, wide), here = min(CHUNK_SLOTS, wide - first);
             whole(b, here);  // runs are a multiple of three slots: the same split between the warps
             if (c + 1 == n && s_tail[di]) rest(reinterpret_cast<const float*>(b + 1280 * (size_t)here));
             if (c + 1 < n) {
@@ -879,11 +880,14 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
       team_sync(team);
       if (mode == 1) stage_issue();
       if (3 * dp + ti < 3 * dn) {
-        const float f = (float)(part[ti] + part[96 + ti] + part[192 + ti]);
+        Acc y = part[ti];
+#pragma unroll
+        for (int u = 1; u < TW; ++u) y += part[96 * u + ti];
+        const float f = (float)y;
         az[3 * dp + ti] = f;
         acc += (Acc)xsc(3 * dp + ti) * (Acc)f;
       }
-      if (di + RS_TEAMS < nD) team_sync(team);
+      if (di + TEAMS < nD) team_sync(team);
     }
     for (uint32_t l = tid; l < nlive; l += RS_THREADS) {
       Acc y0 = 0, y1 = 0, y2 = 0;
@@ -905,7 +909,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
     float* rd = reinterpret_cast<float*>(tscr);
     AA* part = reinterpret_cast<AA*>(tscr + 384);  // [6][32]
     AA* yd = part + 192;
-    for (int di = team; di < nD; di += RS_TEAMS) {
+    for (int di = team; di < nD; di += TEAMS) {
       const uint32_t dp = s_dpos[di], m = 3 * (s_dpos[di + 1] - dp), e = 3 * dp + ti;
       const int T = ((int)m + 31) >> 5;
       const TS* w = nullptr;
@@ -915,7 +919,8 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
                    : (s_tofs[di] != RS_EMPTY ? reinterpret_cast<const TS*>(smem + s_tofs[di])
                                              : (const TS*)S.fac + S.fac_off[d0 + di]);
       }
-      // warp q's tiles are tiles q and q + 3 (zero past the domain's: one code path for all)
+      // warp q's tiles are tiles q and (teams of three) q + 3, zero past the domain's: one code path
+      // for all
       TileRegs<AA, TS> ta, tb;
       auto load = [&](TileRegs<AA, TS>& t, int at) {
         if (at < T * (T + 1) / 2)
@@ -925,7 +930,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
       };
       if (SCH && sizeof(TS) == 2) {  // in registers for both passes
         load(ta, q);
-        load(tb, q + 3);
+        if (TW == 3) load(tb, q + 3);
       }
       float r = 0.f, p = 0.f;
       if ((uint32_t)ti < m) {
@@ -940,7 +945,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
         }
         rv[e] = r;
       }
-      rd[ti] = r;
+      if (TW == 3 || ti < 96) rd[ti] = r;
       team_sync(team);
       if (staged) stage_issue();  // the tiles are in registers
       float zi = 0.f;
@@ -948,12 +953,15 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
         int at;
         if (sizeof(TS) == 4) load(ta, q);
         AA v = ta.rows(rd + 32 * rs_tile_j(q), lane, at);
-        if (sizeof(TS) == 4) load(tb, q + 3);
-        AA v2 = tb.rows(rd + 32 * rs_tile_j(q + 3), lane, at);
+        AA v2 = 0;
+        if (TW == 3) {
+          if (sizeof(TS) == 4) load(tb, q + 3);
+          v2 = tb.rows(rd + 32 * rs_tile_j(q + 3), lane, at);
+        }
         part[32 * q + at] = v;
-        part[32 * (q + 3) + at] = v2;
+        if (TW == 3) part[32 * (q + 3) + at] = v2;
         team_sync(team);
-        {  // y of tile row q: its tiles' partials in storage order
+        if (TW == 3 || q < 3) {  // y of tile row q: its tiles' partials in storage order
           const AA* pr = part + 32 * (q * (q + 1) / 2) + lane;
           AA y = pr[0];
           if (q > 0) y += pr[32];
@@ -961,14 +969,16 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
           yd[ti] = y;
         }
         team_sync(team);
-        if (sizeof(TS) == 4) load(ta, q);
+        if (sizeof(TS) == 4 && (TW == 3 || sizeof(AA) == 8)) load(ta, q);
         v = ta.cols(yd + 32 * rs_tile_i(q), lane, at);
-        if (sizeof(TS) == 4) load(tb, q + 3);
-        v2 = tb.cols(yd + 32 * rs_tile_i(q + 3), lane, at);
+        if (TW == 3) {
+          if (sizeof(TS) == 4) load(tb, q + 3);
+          v2 = tb.cols(yd + 32 * rs_tile_i(q + 3), lane, at);
+        }
         part[32 * q + at] = v;
-        part[32 * (q + 3) + at] = v2;
+        if (TW == 3) part[32 * (q + 3) + at] = v2;
         team_sync(team);
-        {  // z of tile column q
+        if (TW == 3 || q < 3) {  // z of tile column q
           AA z = part[32 * (q * (q + 1) / 2 + q) + lane];
           if (q < 2) z += part[32 * ((q + 1) * (q + 2) / 2 + q) + lane];
           if (q < 1) z += part[32 * 3 + lane];
@@ -1108,38 +1118,19 @@ bool resident_domains(const mguso_schwarz& s, RsRun& run) {
   return d == s.ndom;
 }
 
-static void* resident_kernel(int precond, bool mixed, bool half) {
-  if (precond == MGUSO_PRECOND_BLOCK_JACOBI)
-    return mixed ? (void*)k_pcg_resident<MGUSO_PRECOND_BLOCK_JACOBI, double, float>
-                 : (void*)k_pcg_resident<MGUSO_PRECOND_BLOCK_JACOBI, float, float>;
+template <int TW>
+static void* resident_kernel(bool mixed, bool half) {
   if (half)
-    return mixed ? (void*)k_pcg_resident<MGUSO_PRECOND_SCHWARZ, double, __half>
-                 : (void*)k_pcg_resident<MGUSO_PRECOND_SCHWARZ, float, __half>;
-  return mixed ? (void*)k_pcg_resident<MGUSO_PRECOND_SCHWARZ, double, float>
-               : (void*)k_pcg_resident<MGUSO_PRECOND_SCHWARZ, float, float>;
+    return mixed ? (void*)k_pcg_resident<MGUSO_PRECOND_SCHWARZ, double, __half, TW>
+                 : (void*)k_pcg_resident<MGUSO_PRECOND_SCHWARZ, float, __half, TW>;
+  return mixed ? (void*)k_pcg_resident<MGUSO_PRECOND_SCHWARZ, double, float, TW>
+               : (void*)k_pcg_resident<MGUSO_PRECOND_SCHWARZ, float, float, TW>;
 }
 
 int pcg_resident(const RsSystem& sys, RsWork& w, const RsRun& run, float* x, uint32_t active, float tol,
                  uint32_t max_iter, FusedInst* out, cudaStream_t st) {
   const uint32_t K = run.ninst;
   MG_CHECK_ARG(K >= 1 && K <= PCG_MAX_INST, "resident PCG: 1..8 instances");
-  void* fn = resident_kernel(run.precond, run.mixed, run.half);
-  if (w.fn != fn) {
-    w.fn = nullptr;
-    w.smem = 0;
-    int dev = 0, optin = 0, per_sm = 0;
-    cudaFuncAttributes fa;
-    MG_CUDA(cudaGetDevice(&dev));
-    MG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    MG_CUDA(cudaFuncGetAttributes(&fa, fn));
-    const int dyn = (optin - (int)fa.sharedSizeBytes) / 128 * 128;
-    if (dyn > 0 && cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) == cudaSuccess &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, RS_THREADS, dyn) == cudaSuccess && per_sm >= 1)
-      w.smem = (uint32_t)dyn;
-    cudaGetLastError();
-    w.fn = fn;
-  }
-  if (!w.smem) return MGUSO_ERR_UNSUPPORTED;
   // CTAs per active instance: one each, then one at a time to the instance with the most domains
   // per CTA, until the SMs or the domains run out
   RsArgs a{};
@@ -1181,16 +1172,45 @@ int pcg_resident(const RsSystem& sys, RsWork& w, const RsRun& run, float* x, uin
     a.inst[best].ncta++;
     ++used;
   }
-  uint32_t grid = 0;
+  uint32_t grid = 0, most = 0;  // most: domains of a CTA
   for (uint32_t i = 0; i < a.nrun; ++i) {
-    RsInst& I = a.inst[i];
-    I.cta0 = grid;
-    grid += I.ncta;
+    a.inst[i].cta0 = grid;
+    grid += a.inst[i].ncta;
+    most = std::max(most, ceil_div(nd[i], a.inst[i].ncta));
+  }
+  // Schwarz: teams of six warps, a domain each, where three teams are enough. Time in the solves, three
+  // -> six warps: 64 x 64 grid (one domain per CTA) 1.13 -> 0.97 ms, 100 x 100 (two or three) 2.05 ->
+  // 1.89, a 64 x 64 sheet's step 3.89 -> 3.45; with four domains per CTA three teams take two
+  // turns. Block Jacobi has no tiles to share and loses (100 x 100: 2.70 -> 2.76).
+  const int wide = run.precond == MGUSO_PRECOND_SCHWARZ && most <= 3 ? 1 : 0;
+  void* fn = run.precond == MGUSO_PRECOND_BLOCK_JACOBI
+                 ? (run.mixed ? (void*)k_pcg_resident<MGUSO_PRECOND_BLOCK_JACOBI, double, float, 3>
+                              : (void*)k_pcg_resident<MGUSO_PRECOND_BLOCK_JACOBI, float, float, 3>)
+             : wide ? resident_kernel<6>(run.mixed, run.half)
+                    : resident_kernel<3>(run.mixed, run.half);
+  if (w.fn[wide] != fn) {
+    w.fn[wide] = nullptr;
+    w.smem[wide] = 0;
+    int dev = 0, optin = 0, per_sm = 0;
+    cudaFuncAttributes fa;
+    MG_CUDA(cudaGetDevice(&dev));
+    MG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    MG_CUDA(cudaFuncGetAttributes(&fa, fn));
+    const int dyn = (optin - (int)fa.sharedSizeBytes) / 128 * 128;
+    if (dyn > 0 && cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) == cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, RS_THREADS, dyn) == cudaSuccess && per_sm >= 1)
+      w.smem[wide] = (uint32_t)dyn;
+    cudaGetLastError();
+    w.fn[wide] = fn;
+  }
+  const uint32_t smem = w.smem[wide];
+  if (!smem) return MGUSO_ERR_UNSUPPORTED;
+  for (uint32_t i = 0; i < a.nrun; ++i) {
+    const RsInst& I = a.inst[i];
     const uint32_t dom = ceil_div(nd[i], I.ncta), dia = 32 * ceil_div(I.dd1 - I.dd0, I.ncta);
     // the vectors of a CTA's vertices, the halo and the hash table have to fit
-    const uint64_t need =
-        RS_TEAMS * RS_TEAM_BYTES + 52ull * 32 * dom + 20ull * RS_MAX_HALO + 52ull * dia + 64 + RS_HASH_BYTES;
-    if (dom > (uint32_t)RS_MAX_DOM || need > w.smem) return MGUSO_ERR_UNSUPPORTED;
+    const uint64_t need = RS_SCRATCH + 52ull * 32 * dom + 20ull * RS_MAX_HALO + 52ull * dia + 64 + RS_HASH_BYTES;
+    if (dom > (uint32_t)RS_MAX_DOM || need > smem) return MGUSO_ERR_UNSUPPORTED;
   }
   // records and published sums carry epochs: cleared when allocated and when the epochs run out
   const size_t nrec = 2 * (size_t)std::max<uint32_t>(run.nv, 1), nsum = 3 * (size_t)RS_MAX_G;
@@ -1220,12 +1240,12 @@ int pcg_resident(const RsSystem& sys, RsWork& w, const RsRun& run, float* x, uin
   a.out = out;
   a.tol = tol;
   a.max_iter = max_iter;
-  a.smem_bytes = w.smem;
+  a.smem_bytes = smem;
   w.epoch += span;
   k_rs_reset<<<64, 256, 0, st>>>(a.count, out, K, x, 3 * run.nv);
   MG_CUDA(cudaGetLastError());
   void* args[] = {(void*)&a};
-  MG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(RS_THREADS), args, w.smem, st));
+  MG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(RS_THREADS), args, smem, st));
   return MGUSO_OK;
 }
 
