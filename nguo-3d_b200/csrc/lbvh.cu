@@ -327,10 +327,12 @@ __device__ __forceinline__ int kdelta(const K* __restrict__ keys, int n, int i, 
     return __clz((int)x);
 }
 
+constexpr int RF_THREADS = 256;  // leaves of a subtree that the refit takes whole
+
 template <class K>
 __global__ void k_karras(const K* __restrict__ keys, uint32_t nn, uint32_t* __restrict__ parent_int,
                          uint32_t* __restrict__ parent_leaf, uint32_t* __restrict__ range_end,
-                         uint32_t* __restrict__ flags) {
+                         uint32_t* __restrict__ flags, uint32_t* __restrict__ roots, uint32_t* __restrict__ nroots) {
   const int n = (int)nn;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n - 1) return;
@@ -363,36 +365,36 @@ __global__ void k_karras(const K* __restrict__ keys, uint32_t nn, uint32_t* __re
   else
     parent_int[g + 1] = (uint32_t)i | RIGHT_BIT;
   if (i == 0) parent_int[0] = NO_PARENT;
+  // the children that a refit's CTA can take whole
+  if (last - first >= RF_THREADS) {
+    const bool l = g - first < RF_THREADS, r = last - g <= RF_THREADS;
+    if (l || r) {
+      uint32_t at = atomicAdd(nroots, (uint32_t)l + (uint32_t)r);
+      if (l) roots[at++] = (uint32_t)g | (first == g ? LEAF_BIT : 0u);
+      if (r) roots[at] = (uint32_t)(g + 1) | (last == g + 1 ? LEAF_BIT : 0u);
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------------------
 // Boxes: one climb per leaf (in sorted order), which writes its box into its half of the parent's
 // record; the second to arrive at a node goes on with the union of both halves. `v` is the
-// positions, or the displacements for the CCD's records. A level whose node covers only leaves
-// of this CTA (node i covers the leaves from i to range_end[i]) is crossed in shared memory; the
-// others cost a fence, an atomic and a read of the sibling's half from L2, about 1 us a level.
-// Before -> after (leaf boxes in a kernel of their own, a memset of the flags, children's boxes and
-// indices gathered again at every level): 8 000 to 12 000 primitives 37 -> 26 us, 41 401 50 -> 36,
-// 4 M 570 -> 389 (640 MB are 100).
+// positions, or the displacements for the CCD's records. What bounds a refit is the longest climb:
+// a level across CTAs costs a fence, an atomic and a read of the sibling's half from L2, about 1 us.
+// So CTAs take whole subtrees of up to 256 leaves (found with the tree: the largest such subtrees,
+// listed in any order) and climb them in shared memory; only the tree above them is climbed
+// through L2. Before -> after (leaf boxes in a kernel of their own, a memset of the flags,
+// children's boxes and indices gathered again at every level), in brackets with CTAs of 256
+// consecutive leaves, whose blocks cut subtrees at every level: 8 000 to 12 000 primitives
+// 37 -> 15 (26) us, 41 401 50 -> 24 (36), 4.2 M 570 -> 340 (389; 640 MB are 100).
 // ---------------------------------------------------------------------------------------
-constexpr int RF_THREADS = 256;
-
-__global__ void __launch_bounds__(RF_THREADS) k_refit(const float* __restrict__ v, const uint32_t* __restrict__ tris,
-                                                      const uint32_t* __restrict__ perm,
-                                                      const uint32_t* __restrict__ parent_leaf,
-                                                      const uint32_t* __restrict__ parent_int,
-                                                      const uint32_t* __restrict__ range_end, float4* rec,
-                                                      uint32_t* flags, uint32_t nt) {
-  __shared__ uint32_t s_par[RF_THREADS], s_end[RF_THREADS], s_flag[RF_THREADS];
-  __shared__ float s_box[2][6][RF_THREADS];
-  const uint32_t tid = threadIdx.x, b0 = blockIdx.x * RF_THREADS, i = b0 + tid;
-  if (i + 1 < nt) {
-    s_par[tid] = parent_int[i];
-    s_end[tid] = range_end[i];
-  }
-  s_flag[tid] = 0;
-  __syncthreads();
-  if (i >= nt) return;
+__device__ __forceinline__ void refit_climb(const float* __restrict__ v, const uint32_t* __restrict__ tris,
+                                            const uint32_t* __restrict__ perm,
+                                            const uint32_t* __restrict__ parent_leaf,
+                                            const uint32_t* __restrict__ parent_int, float4* rec, uint32_t* flags,
+                                            uint32_t nt, uint32_t b0, uint32_t top, const uint32_t* s_par,
+                                            uint32_t* s_flag, float (*s_box)[6][RF_THREADS]) {
+  const uint32_t i = b0 + threadIdx.x;
   const uint32_t t = perm[i];
   const uint32_t v0 = tris[3 * t], v1 = tris[3 * t + 1], v2 = tris[3 * t + 2];
   float lo[3], hi[3];
@@ -411,19 +413,23 @@ __global__ void __launch_bounds__(RF_THREADS) k_refit(const float* __restrict__ 
     return;
   }
   uint32_t id = i | LEAF_BIT, up = parent_leaf[i];
+  bool local = true;
   while (up != NO_PARENT) {
-    const uint32_t p = up & ~RIGHT_BIT, side = up >> 31, l = p - b0;
+    local = local && up != top;
+    const uint32_t p = up & ~RIGHT_BIT, side = up >> 31;
     float4* half = rec + 4 * (size_t)p + 2 * side;
     __stcg(half, make_float4(lo[0], lo[1], lo[2], __uint_as_float(id)));
     __stcg(half + 1, make_float4(hi[0], hi[1], hi[2], 0.f));
-    if (l < RF_THREADS && s_end[l] - b0 < RF_THREADS) {
+    if (local) {
+      const uint32_t l = p - b0;
+      if (l >= RF_THREADS) return;  // not of a tree: the sort gave up (its status says so)
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         s_box[side][c][l] = lo[c];
         s_box[side][3 + c][l] = hi[c];
       }
       __threadfence_block();
-      if (atomicAdd(&s_flag[l], 1u) == 0u) return;
+      if (!(atomicAdd(&s_flag[l], 1u) & 1u)) return;
       __threadfence_block();
       volatile const float(*o)[RF_THREADS] = s_box[side ^ 1];
 #pragma unroll
@@ -448,6 +454,34 @@ __global__ void __launch_bounds__(RF_THREADS) k_refit(const float* __restrict__ 
       up = next;
     }
     id = p;
+  }
+}
+
+__global__ void __launch_bounds__(RF_THREADS, 8) k_refit(const float* __restrict__ v, const uint32_t* __restrict__ tris,
+                                                      const uint32_t* __restrict__ perm,
+                                                      const uint32_t* __restrict__ parent_leaf,
+                                                      const uint32_t* __restrict__ parent_int,
+                                                      const uint32_t* __restrict__ range_end,
+                                                      const uint32_t* __restrict__ roots,
+                                                      const uint32_t* __restrict__ nroots, float4* rec,
+                                                      uint32_t* flags, uint32_t nt) {
+  __shared__ uint32_t s_par[RF_THREADS], s_flag[RF_THREADS];
+  __shared__ float s_box[2][6][RF_THREADS];
+  const uint32_t tid = threadIdx.x;
+  const bool whole = nt <= RF_THREADS;
+  const uint32_t nr = whole ? 1u : *nroots;
+  for (uint32_t at = blockIdx.x; at < nr; at += gridDim.x) {
+    // this subtree: leaves b0 .. b0 + count - 1, inner nodes within the same indices
+    const uint32_t root = whole ? (nt == 1 ? LEAF_BIT : 0u) : roots[at], ri = root & ~LEAF_BIT;
+    const uint32_t re = (root & LEAF_BIT) ? ri : range_end[ri], b0 = min(ri, re), count = max(ri, re) - b0 + 1;
+    const uint32_t top = whole ? NO_PARENT : ((root & LEAF_BIT) ? parent_leaf[ri] : parent_int[ri]);
+    __syncthreads();
+    if (tid < count) {
+      s_par[tid] = parent_int[b0 + tid];
+      s_flag[tid] = 0;
+    }
+    __syncthreads();
+    if (tid < count) refit_climb(v, tris, perm, parent_leaf, parent_int, rec, flags, nt, b0, top, s_par, s_flag, s_box);
   }
 }
 
@@ -600,23 +634,30 @@ int radix_sort_pairs(Lbvh* b, void* keys, uint32_t* vals, uint32_t n, int key_bi
 }
 
 // the centroid-bounds accumulator's start (ordered bits): the three minima at their highest
-// value, the three maxima at their lowest
-__global__ void k_ord_init(uint32_t* __restrict__ ord) {
+// value, the three maxima at their lowest; and the count of the refit's subtrees
+__global__ void k_ord_init(uint32_t* __restrict__ ord, uint32_t* __restrict__ nroots) {
+  if (threadIdx.x == 0) *nroots = 0;
   if (threadIdx.x < 6) ord[threadIdx.x] = threadIdx.x < 3 ? 0xffffffffu : 0u;
 }
 
 static int lbvh_reserve_nodes(Lbvh* b, uint32_t nt) {
   const size_t nn = std::max<uint32_t>(nt, 2);
-  MG_TRY(b->parent_int.reserve(nn));
-  MG_TRY(b->parent_leaf.reserve(nn));
-  MG_TRY(b->range_end.reserve(nn));
-  MG_TRY(b->rec.reserve(4 * nn));
-  return b->flags.reserve(nn);
+  MG_TRY(b->shape.reserve(6 * nn + 1));
+  b->parent_int = b->shape.p;
+  b->parent_leaf = b->parent_int + nn;
+  b->range_end = b->parent_leaf + nn;
+  b->flags = b->range_end + nn;
+  b->roots = b->flags + nn;  // at most nt of a tree; two per node whatever the keys
+  b->nroots = b->roots + 2 * nn;
+  return b->rec.reserve(4 * nn);
 }
 
 static int launch_refit(Lbvh* b, const float* v, const uint32_t* tris, float4* rec, cudaStream_t s) {
-  k_refit<<<ceil_div(b->nt, RF_THREADS), RF_THREADS, 0, s>>>(v, tris, b->perm.p, b->parent_leaf.p, b->parent_int.p,
-                                                            b->range_end.p, rec, b->flags.p, b->nt);
+  // the subtrees' number is known on the device only: on average more than 64 leaves each. One per CTA,
+  // so that the climbs above them overlap with the next (resident CTAs in a loop: 4.2 M 620 us).
+  const uint32_t grid = b->nt <= RF_THREADS ? 1u : ceil_div(b->nt, 64);
+  k_refit<<<grid, RF_THREADS, 0, s>>>(v, tris, b->perm.p, b->parent_leaf, b->parent_int, b->range_end, b->roots,
+                                      b->nroots, rec, b->flags, b->nt);
   MG_CUDA(cudaGetLastError());
   return MGUSO_OK;
 }
@@ -633,7 +674,7 @@ static int build_impl(Lbvh* b, const float* pos, const uint32_t* tris, uint32_t 
   MG_TRY(b->ord.reserve(8));
   MG_TRY(b->status.reserve(4));
   if (nt == 0) return MGUSO_OK;
-  k_ord_init<<<1, 32, 0, s>>>(b->ord.p);
+  k_ord_init<<<1, 32, 0, s>>>(b->ord.p, b->nroots);
   int sms = device_sm_count();
   k_centroid_bounds<<<std::min<uint32_t>(ceil_div(nt, 256), sms * 8), 256, 0, s>>>(pos, tris, nt, b->ord.p);
   k_bounds_finish<<<1, 32, 0, s>>>(b->ord.p, b->params.p);
@@ -644,8 +685,8 @@ static int build_impl(Lbvh* b, const float* pos, const uint32_t* tris, uint32_t 
   MG_TRY(sort_impl<K>(b, keys, b->perm.p, nt, key_bits, s));
   if (b->ev_on) cudaEventRecord(b->ev[2], s);
   if (nt > 1) {
-    k_karras<K><<<ceil_div(nt - 1, 256), 256, 0, s>>>(keys, nt, b->parent_int.p, b->parent_leaf.p, b->range_end.p,
-                                                     b->flags.p);
+    k_karras<K><<<ceil_div(nt - 1, 256), 256, 0, s>>>(keys, nt, b->parent_int, b->parent_leaf, b->range_end,
+                                                     b->flags, b->roots, b->nroots);
   }
   if (b->ev_on) cudaEventRecord(b->ev[3], s);
   MG_TRY(launch_refit(b, pos, tris, b->rec.p, s));

@@ -15,16 +15,19 @@ struct Lbvh {
   bool shaped = false;              // the last build enqueued its whole shape (refits may follow)
   DevBuf<unsigned char> keys;       // nt keys (u32 or u64), sorted after build
   DevBuf<uint32_t> perm;            // sorted leaf -> triangle
-  // per inner node, its parent and its range's other end (its own index is one end); a parent's
-  // top bit says that the child is its right one
-  DevBuf<uint32_t> parent_int, parent_leaf, range_end;
+  // the shape, in one allocation: per inner node, its parent (the top bit says that it is the right
+  // child), its range's other end (its own index is one end) and the arrivals at it (0 after a build's
+  // shape, even after each refit); per leaf, its parent; the refit's subtrees: their roots
+  // (LEAF_BIT for a leaf) and number
+  DevBuf<uint32_t> shape;
+  uint32_t *parent_int = nullptr, *parent_leaf = nullptr, *range_end = nullptr, *flags = nullptr, *roots = nullptr,
+           *nroots = nullptr;
   // Per inner node, one 64-byte record of its two children: (lo, id), (hi, -), of the left, then of
   // the right one, id the child's index with LEAF_BIT for a leaf (as float bits), so that a walk
   // reads a node's children and their boxes in one round of loads. A one-primitive tree has one
   // record, its right child empty (NaN: never entered). drec: the same of the displacement boxes
   // (CCD pruning).
   DevBuf<float4> rec, drec;
-  DevBuf<uint32_t> flags;           // arrivals at a node: 0 after a build's shape, even after each refit
   DevBuf<float> params;             // centroid lo.xyz, inv.xyz
   DevBuf<uint32_t> ord;
   DevBuf<uint32_t> status;
