@@ -634,7 +634,8 @@ def run_batch(args, dist: Dist):
             "frac": round(achieved / peak, 4),
             "traffic": None if traffic is None else int(traffic),
             "traffic_source": tsrc, "peak_kind": f"{peak_kind} (burst copy)",
-            "kernel": kname + " (fused PCG, timed inside a solve of the last Newton system)",
+            "kernel": kname + " (fused PCG, the path of systems that the resident PCG cannot hold, timed "
+                      "inside a solve of the last Newton system; the timed steps solve in k_pcg_resident)",
             "us_per_launch": round(us, 2), "bytes_per_launch": int(nbytes),
             "fused": {k: {"kernel": knames[k], "us": round(v[0], 2), "bytes": int(v[1]),
                           "GB/s": round(v[1] / (v[0] * 1e-6) / 1e9, 1)} for k, v in fused.items()},
