@@ -489,15 +489,19 @@ __global__ void __launch_bounds__(RF_THREADS, 8) k_refit(const float* __restrict
 // Point queries: a warp takes 32 of them, neighbours in Morton order (qorder), down the tree
 // together (warp_walk) and appends the pairs it finds 32 at a time, so that the pair counter takes
 // one atomic per 32 pairs. 12.6 M points over 4.2 M triangles, before -> after (one stack per
-// lane, boxes and child indices in separate arrays, one atomic per pair): 3.42 -> 2.50 ms (2.73
-// with all walks from the root), and 0.10 ms for the query boxes, now made in registers.
+// lane, boxes and child indices in separate arrays, one atomic per pair): 3.42 -> 2.13 ms, and 0.10
+// ms for the query boxes, now made in registers. With all walks from the root 2.73. What bounds
+// it is L1: 32 lanes on different nodes gather 64 bytes each. So the queues are short, which
+// leaves L1 more of the SM's memory than the scenes' of 1 024 nodes would (2.50 ms; 256 nodes: no better).
 // ---------------------------------------------------------------------------------------
+constexpr int PT_CAP = 384;  // queued nodes per warp
+
 __global__ void __launch_bounds__(WQ_WARPS * 32) k_traverse(BvhSet bv, const float* __restrict__ pts, float pad,
                                                             const uint32_t* __restrict__ qorder, uint32_t nq,
                                                             uint32_t per, uint32_t* __restrict__ pairs, uint64_t cap,
                                                             unsigned long long* __restrict__ count,
                                                             uint32_t* __restrict__ status) {
-  __shared__ WalkMem<BoxQuery> mem[WQ_WARPS];
+  __shared__ WalkMem<BoxQuery, PT_CAP> mem[WQ_WARPS];
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, first = (blockIdx.x * WQ_WARPS + w) * per;
   const uint32_t k = first + lane;
   const bool valid = lane < per && k < nq;

@@ -140,16 +140,16 @@ inline BvhView lbvh_view(const Lbvh& b) { return BvhView{b.perm.p, b.rec.p, b.dr
 // minima and sums, and the leaves reached do not depend on the order of the tests.
 constexpr int WQ_WARPS = 4;   // 128-thread blocks
 constexpr int WQ_QCAP = 96;   // < 32 left over + 2 leaves per lane and round
-// queued nodes per warp: a round adds at most 32; past FW_FULL one node is taken at a time, which
-// goes down depth first and adds at most one per level
-constexpr int FW_CAP = 1024, FW_FULL = FW_CAP - 128;
+// queued nodes per warp: a round adds at most 32; with FW_SPARE places left one node is taken at a
+// time, which goes down depth first and adds at most one per level
+constexpr int FW_CAP = 1024, FW_SPARE = 128;
 
-template <class Q>
+template <class Q, int CAP = FW_CAP>
 struct WalkMem {  // shared memory of one warp
   Q query[32];
-  uint32_t node[FW_CAP];
+  uint32_t node[CAP];
   uint2 pair[WQ_QCAP];
-  uint8_t slot[FW_CAP];
+  uint8_t slot[CAP];
   uint8_t inst[32];
 };
 
@@ -178,8 +178,8 @@ __device__ __forceinline__ void wq_take(uint2* q, int& n, int min_n, F&& solve) 
 // numbered first + l. keep(slot, primitive) says whether a leaf reached is to be solved. The walks
 // begin at node `start` (0, the root, or one that covers all that the queries can meet).
 // Returns false when the node queue overflowed.
-template <class Q, class KEEP, class SOLVE>
-__device__ __forceinline__ bool warp_walk(WalkMem<Q>& m, const BvhSet& bs, uint32_t first, bool valid, uint32_t k,
+template <class Q, int CAP, class KEEP, class SOLVE>
+__device__ __forceinline__ bool warp_walk(WalkMem<Q, CAP>& m, const BvhSet& bs, uint32_t first, bool valid, uint32_t k,
                                           const Q& mine, KEEP&& keep, SOLVE&& solve, uint32_t start = 0) {
   const int lane = (int)(threadIdx.x & 31);
   const unsigned below = (1u << lane) - 1u;
@@ -201,8 +201,8 @@ __device__ __forceinline__ bool warp_walk(WalkMem<Q>& m, const BvhSet& bs, uint3
   }
   __syncwarp();
   while (n > 0) {
-    const int take = n <= FW_FULL ? min(n, 32) : 1;
-    if (n + take > FW_CAP) {
+    const int take = n <= CAP - FW_SPARE ? min(n, 32) : 1;
+    if (n + take > CAP) {
       ok = false;
       break;
     }

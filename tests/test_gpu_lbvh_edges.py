@@ -59,3 +59,23 @@ def test_point_queries_at_warp_edges(ctx, npts, offset):
     assert b.status() == 0 and int(cnt.item()) == len(want)
     got = buf[offset:offset + 2 * len(want)].cpu().numpy().reshape(-1, 2)
     assert sorted(map(tuple, got.tolist())) == sorted(want)
+
+
+@pytest.mark.parametrize("nt,npts", [(2, 40), (500, 33), (3000, 64)])
+def test_queries_that_meet_everything(ctx, nt, npts):
+    """Every point meets every triangle, so the walks' node queues fill up and go on node by node."""
+    pos, tris = scenes.triangle_soup(nt, seed=11)
+    pts = np.concatenate([pos, pos])[:npts] if pos.shape[0] >= npts else np.resize(pos, (npts, 3))
+    import torch
+    b = lbvh.Lbvh(ctx)
+    s = torch.cuda.current_stream().cuda_stream
+    pd, td, qd = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (pos, tris.astype(np.int32), pts))
+    b.build(pd.data_ptr(), pos.shape[0], td.data_ptr(), nt, 30, s)
+    cap = nt * npts
+    buf = torch.full((cap, 2), -1, dtype=torch.int32, device="cuda")
+    cnt = torch.zeros(1, dtype=torch.int64, device="cuda")
+    b.query_points(qd.data_ptr(), npts, 10.0, buf.data_ptr(), cap, cnt.data_ptr(), s)
+    torch.cuda.synchronize()
+    assert b.status() == 0 and int(cnt.item()) == cap
+    key = buf.cpu().numpy().astype(np.int64)
+    assert np.array_equal(np.sort(key[:, 0] * nt + key[:, 1]), np.arange(cap))
