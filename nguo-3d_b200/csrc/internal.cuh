@@ -210,11 +210,7 @@ struct RsRun {
   bool mixed = true, half = false;
   int sms = 148;
   uint32_t nv = 0, ninst = 1;
-  const mguso_bsr* a = nullptr;  // the pattern and the domains, on the host
-  const mguso_schwarz* sw = nullptr;
-  // of a CTA's blocks, how many in a thousand may find no place packed before the solve is left to
-  // the other PCG (resident_walked)
-  uint32_t walked_max = 0;
+  uint64_t nnz = 0;  // blocks of A
   uint32_t vert[PCG_MAX_INST + 1] = {}, dom[PCG_MAX_INST + 1] = {}, diag[PCG_MAX_INST] = {};
 };
 
@@ -228,15 +224,12 @@ struct RsWork {
   DevBuf<uint4> sums;
   DevBuf<uint32_t> count;
   uint32_t epoch = 0;  // epochs used so far
-  // per instance, CTAs it was found to run well on (so it does on more) and not to (so on fewer)
-  uint32_t good[PCG_MAX_INST] = {}, poor[PCG_MAX_INST] = {};
 };
 
 // Solves the instances of `active` into x (3 floats per vertex; the others get x = 0) and
 // their results into out[k] (device), enqueued on st without a host wait. Returns
 // MGUSO_ERR_UNSUPPORTED, having enqueued nothing, when the system's vectors do not fit in the
-// SMs' shared memory (beyond about 64 domains or 2 000 vertices per SM) or too many of its blocks
-// have no place beside them.
+// SMs' shared memory (beyond about 64 domains or 2 000 vertices per SM).
 int pcg_resident(const RsSystem& sys, RsWork& w, const RsRun& run, float* x, uint32_t active, float tol,
                  uint32_t max_iter, FusedInst* out, cudaStream_t st);
 
