@@ -39,6 +39,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "recip.cuh"
 #include "reduce.cuh"
 #include "scene.cuh"
 #include "tiles.cuh"
@@ -126,14 +127,6 @@ __device__ __forceinline__ void st_rlx(void* p, uint4 v) {
 __device__ __forceinline__ void st_rec(float4* p, float x, float y, float z, uint32_t epoch) {
   st_rlx(p, make_uint4(__float_as_uint(x), __float_as_uint(y), __float_as_uint(z), epoch));
 }
-// 1 / v by Newton steps on the hardware's approximation, to a unit in the last place
-__device__ __forceinline__ double rs_rcp(double v) {
-  double x;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(v));
-  x = fma(x, fma(-v, x, 1.0), x);
-  return fma(x, fma(-v, x, 1.0), x);
-}
-
 // ---- a 32 x 32 tile held by a warp in registers -------------------------------------------
 // Both passes of z = W^T (W r) run from one load of the tile: a warp reads it as whole 512-byte
 // rows (no bank conflicts, full sectors from L2), every lane multiplies what it holds, and
@@ -1053,7 +1046,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
           s_done = 1;
           s_status = ST_PCG_BREAKDOWN;
         } else {
-          s_alpha = (float)(s_rz * rs_rcp(t0));
+          s_alpha = (float)quotient(s_rz, t0);  // a p.Ap that overflowed takes no step
         }
       }
       __syncthreads();
@@ -1073,7 +1066,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
       } else if (it >= a.max_iter || (t0 <= s_lim2 && sqrt(t0) / s_bnorm <= (double)a.tol)) {
         s_done = 1;  // the residual itself is only formed where it can be within the tolerance
       } else {
-        s_beta = (float)(t1 * rs_rcp(s_rz));
+        s_beta = (float)quotient(t1, s_rz);
         s_rz = t1;
       }
     }

@@ -23,6 +23,7 @@
 #include <algorithm>
 
 #include "internal.cuh"
+#include "recip.cuh"
 #include "tiles.cuh"
 
 namespace mg {
@@ -50,14 +51,6 @@ __host__ __device__ constexpr int fc_smem_bytes() {
   constexpr int T = (8 * NB + 31) / 32;
   constexpr int block = 8 * NB * fc_ld<NB>() * 4, tiles = T * (T + 1) / 2 * TILE_FLOATS * 4;
   return block > tiles ? block : tiles;
-}
-
-// 1 / p by Newton steps on the hardware's approximation (two double the correct bits past 53)
-__device__ __forceinline__ double fc_rcp(double p) {
-  double x;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(p));
-  x = fma(x, fma(-p, x, 1.0), x);
-  return fma(x, fma(-p, x, 1.0), x);
 }
 
 __device__ __forceinline__ double fc_block_sum(double v, double* s2) {
@@ -124,7 +117,7 @@ __device__ void fc_factor_store(float* sm, int m, TS* __restrict__ out, float* s
         break;
       }
       if (tid == 0) s_piv[k] = p;
-      const double w = fc_rcp(p);
+      const double w = recip(p);  // p > 1e-14; an infinite one fails the next pivot's test
       double u[NB];
 #pragma unroll
       for (int b = 0; b < NB; ++b) u[b] = v[tj + 8 * b];
