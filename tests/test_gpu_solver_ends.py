@@ -36,6 +36,24 @@ def test_overflowing_step_length(ctx):
     assert np.abs(x - want).max() <= 1e-5 * want
 
 
+@pytest.mark.parametrize("precond", ["schwarz", "block"])
+@pytest.mark.parametrize("precision", ["fp32", "mixed"])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_isolated_vertex_with_a_non_finite_block(ctx, precond, precision, bad):
+    """A vertex without neighbours and without a load whose block holds a NaN or an infinity: A p
+    does too, p.Ap is not a number above zero and the solve breaks off before its first step."""
+    nb0, rp0, col0, val0 = scenes.grid_bsr(12, 2)
+    nb = nb0 + 3
+    rp = np.concatenate([rp0, rp0[-1] + 1 + np.arange(3)]).astype(np.uint32)
+    col = np.concatenate([col0, nb0 + np.arange(3)]).astype(np.uint32)
+    val = np.concatenate([val0, np.tile(2 * np.eye(3, dtype=np.float32), (3, 1, 1))])
+    val[-2, 0, 1] = bad
+    b = np.random.default_rng(5).standard_normal((nb, 3)).astype(np.float32)
+    b[nb0:] = 0
+    x, st = solve(ctx, nb, rp, col, val, b.reshape(-1), precond, precision)
+    assert st.iters == 0 and np.all(x == 0)
+
+
 RECIP = r"""
 #include <cmath>
 #include <cstdint>
