@@ -239,8 +239,9 @@ typedef struct {
   uint32_t schwarz_domain;
   int precision;
   int pcg_mode;            /* 0, 2: one cooperative launch per linear solve, the system resident in
-                                 the SMs' shared memory; systems too large for it (beyond about
-                                 64 Schwarz domains or 2 000 vertices per SM) and scenes with a
+                                 the SMs' shared memory; systems whose rows it can neither keep
+                                 nor stage there (beyond about 29 Schwarz domains of 32 vertices,
+                                 or with block Jacobi 650 vertices, per SM) and scenes with a
                                  pcg_variant run two fused kernels per iteration (rows, domains)
                                  at full occupancy, replayed as CUDA graphs;
                               1: one launch per PCG kernel, replayed as CUDA graphs (single

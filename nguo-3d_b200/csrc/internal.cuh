@@ -211,8 +211,13 @@ struct RsRun {
   int sms = 148;
   uint32_t nv = 0, ninst = 1;
   uint64_t nnz = 0;  // blocks of A
+  // of a CTA's blocks, how many in a thousand may have no place packed before the solve is left to
+  // the other PCG (resident_walked)
+  uint32_t walked_max = 0;
   uint32_t vert[PCG_MAX_INST + 1] = {}, dom[PCG_MAX_INST + 1] = {}, diag[PCG_MAX_INST] = {};
 };
+
+constexpr uint32_t WALKED_SCENE = 100, WALKED_SOLVER = 780;  // walked_max: see resident_walked
 
 struct RsWork {
   // per team size: the kernel that `smem` was found for and its dynamic shared memory (0: it cannot
@@ -224,14 +229,17 @@ struct RsWork {
   DevBuf<uint4> sums;
   DevBuf<uint32_t> count;
   uint32_t epoch = 0;  // epochs used so far
+  // per instance, the CTAs that it was found to run well on (it does on more) and not to (nor on fewer)
+  uint32_t good[PCG_MAX_INST] = {}, poor[PCG_MAX_INST] = {};
 };
 
 // Solves the instances of `active` into x (3 floats per vertex; the others get x = 0) and
 // their results into out[k] (device), enqueued on st without a host wait. Returns
 // MGUSO_ERR_UNSUPPORTED, having enqueued nothing, when the system's vectors do not fit in the
-// SMs' shared memory (beyond about 64 domains or 2 000 vertices per SM).
-int pcg_resident(const RsSystem& sys, RsWork& w, const RsRun& run, float* x, uint32_t active, float tol,
-                 uint32_t max_iter, FusedInst* out, cudaStream_t st);
+// SMs' shared memory (beyond about 64 domains or 2 000 vertices per SM) or too many of its blocks
+// have no place beside them. a, sw: its pattern and domains on the host (sw null: block Jacobi).
+int pcg_resident(const RsSystem& sys, const mguso_bsr& a, const mguso_schwarz* sw, RsWork& w, const RsRun& run,
+                 float* x, uint32_t active, float tol, uint32_t max_iter, FusedInst* out, cudaStream_t st);
 
 // Domain ranges per instance of a one-level Schwarz preconditioner whose domains are grouped by
 // instance; false when they are not.

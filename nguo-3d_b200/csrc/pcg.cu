@@ -242,6 +242,8 @@ static int pcg_solve_resident(mguso_linear_solver* s, float tol, uint32_t max_it
     r.sms = s->ctx->sm_count;
     r.nv = a->nb;
     r.nnz = a->nnzb;
+    r.walked_max = WALKED_SOLVER;
+    s->rs.good[0] = s->rs.poor[0] = 0;
     r.vert[1] = a->nb;
     if (sw && !resident_domains(*sw, r)) return MGUSO_ERR_UNSUPPORTED;
     s->rs_ready = true;
@@ -263,7 +265,7 @@ static int pcg_solve_resident(mguso_linear_solver* s, float tol, uint32_t max_it
   }
   MG_TRY(s->rs_inst.reserve(1));
   MG_TRY(s->rs_out.reserve(1));
-  MG_TRY(pcg_resident(y, s->rs, r, s->work.x.p, 1, tol, max_iter, s->rs_inst.p, st));
+  MG_TRY(pcg_resident(y, *a, sw, s->rs, r, s->work.x.p, 1, tol, max_iter, s->rs_inst.p, st));
   MG_CUDA(cudaMemcpyAsync(s->rs_out.p, s->rs_inst.p, sizeof(FusedInst), cudaMemcpyDeviceToHost, st));
   MG_CUDA(cudaStreamSynchronize(st));
   const FusedInst& o = *s->rs_out.p;

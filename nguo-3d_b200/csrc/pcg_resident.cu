@@ -1120,6 +1120,78 @@ bool resident_domains(const mguso_schwarz& s, RsRun& run) {
   return d == s.ndom;
 }
 
+// Of the blocks of one CTA, the largest share (in thousandths, over instance k's CTAs) that would be
+// walked in the BSR because their rows are neither resident nor staged, found as the kernel's set-up
+// places them (without contact blocks, which only the device knows, and isolated vertices, which
+// bear no load in a scene). A walked block costs two polled records, so a chip full of them
+// loses to the other PCGs. us an iteration, walked there or not -> with the other PCG:
+//   scenes, Schwarz, mixed: 300 x 300 sheet (20 domains a CTA, all staged) 24 -> 37; six garments (29,
+//     staged) 31 -> 53; seven (31, the worst CTA walks 78%) 88 -> 60; eight (37, 85%) 102 -> 73;
+//   scenes, block Jacobi: 300 x 300 sheet (20, staged) 20 -> 27; 360 x 360 (28, 79%) 39 -> 29; five
+//     garments (33, 80%) 42 -> 29; 545 x 545 sheet 134 -> 53;
+//   solver, Schwarz, mixed (7 blocks a row): 360 x 360 grid (28, 0%) 45 -> 74; 400 x 400 (34, 65%) 74 -> 84;
+//     440 (41, 76%) 93 -> 95; 460 (45, 80%) 103 -> 99; 480 112 -> 103;
+//   solver, Schwarz, FP32: 400 68 -> 74; 440 87 -> 86; 460 92 -> 84;
+//   solver, block Jacobi, mixed: 460 (45, 78%) 32 -> 35; 480 (49, 82%) 38 -> 38; 545 61 -> 49.
+// The share jumps where the staging buffers (147 KB) no longer fit beside a CTA's vectors. So
+// scenes allow a tenth (WALKED_SCENE), the solver, whose other PCG takes five launches, 78%.
+static uint32_t resident_walked(const mguso_bsr& a, const mguso_schwarz* sw, const RsRun& run, uint32_t k,
+                                uint32_t ncta, uint32_t smem, uint32_t stage) {
+  const uint32_t v0 = run.vert[k], nv = run.vert[k + 1] - v0;
+  const uint32_t dn0 = sw ? run.dom[k] : 0, nd = sw ? run.diag[k] - dn0 : ceil_div(nv, 32);
+  auto dstart = [&](uint32_t d) { return sw ? sw->h_dom_start[dn0 + d] : v0 + std::min(32 * d, nv); };
+  auto vert = [&](uint32_t pos) { return sw ? sw->h_dom_verts[pos] : pos; };
+  auto share = [&](uint32_t j) { return (uint32_t)((uint64_t)nd * j / ncta); };
+  std::vector<uint32_t> owner(nv, ncta), seen(nv, ncta);
+  for (uint32_t j = 0; j < ncta; ++j)
+    for (uint32_t pos = dstart(share(j)); pos < dstart(share(j + 1)); ++pos) owner[vert(pos) - v0] = j;
+  struct Dom {
+    uint64_t bytes, tail;
+    uint32_t blocks;
+  };
+  std::vector<Dom> doms;
+  uint32_t worst = 0;
+  for (uint32_t j = 0; j < ncta; ++j) {
+    uint64_t own = 0, halo = 0, need = 0, blocks = 0, walked = 0;
+    doms.clear();
+    for (uint32_t d = share(j); d < share(j + 1); ++d) {
+      uint32_t len[32] = {}, n = 0;
+      Dom m{0, 0, 0};
+      for (uint32_t pos = dstart(d); pos < dstart(d + 1); ++pos) {
+        const uint32_t v = vert(pos);
+        m.blocks += len[n++] = a.h_row_ptr[v + 1] - a.h_row_ptr[v];
+        for (uint32_t e = a.h_row_ptr[v]; e < a.h_row_ptr[v + 1]; ++e) {
+          const uint32_t c = a.h_col[e] - v0;
+          if (c >= nv || owner[c] == j || seen[c] == j) continue;
+          seen[c] = j;
+          ++halo;
+        }
+      }
+      std::sort(len, len + n, [](uint32_t x, uint32_t y) { return x > y; });
+      const uint32_t wide = len[RS_WIDE - 1];
+      for (uint32_t i = 0; i < n; ++i) m.tail += len[i] - std::min(len[i], wide);
+      m.tail = (40 * m.tail + 15) & ~15ull;
+      m.bytes = 1280ull * wide + m.tail;
+      const uint32_t T = (3 * n + 31) / 32;
+      need += m.bytes + (sw ? (uint64_t)T * (T + 1) / 2 * TILE_FLOATS * (run.half ? 2 : 4) : (36ull * n + 15) & ~15ull);
+      own += n;
+      blocks += m.blocks;
+      doms.push_back(m);
+    }
+    uint64_t cur = RS_SCRATCH + 52 * own + 20 * std::min<uint64_t>(halo, RS_MAX_HALO) + 16;
+    const bool staged = cur + need > smem && cur + stage <= smem;
+    const uint64_t lim = std::min(smem - (staged ? stage : 0u), smem - RS_HASH_BYTES);
+    for (const Dom& m : doms) {
+      if (m.blocks < 60000u && cur + m.bytes <= lim)
+        cur += m.bytes;
+      else if (!(m.blocks < 60000u && staged && m.tail <= RS_CHUNK))
+        walked += m.blocks;
+    }
+    worst = std::max(worst, (uint32_t)(1000 * walked / std::max<uint64_t>(blocks, 1)));
+  }
+  return worst;
+}
+
 template <int TW>
 static void* resident_kernel(bool mixed, bool half) {
   if (half)
@@ -1129,8 +1201,8 @@ static void* resident_kernel(bool mixed, bool half) {
                : (void*)k_pcg_resident<MGUSO_PRECOND_SCHWARZ, float, float, TW>;
 }
 
-int pcg_resident(const RsSystem& sys, RsWork& w, const RsRun& run, float* x, uint32_t active, float tol,
-                 uint32_t max_iter, FusedInst* out, cudaStream_t st) {
+int pcg_resident(const RsSystem& sys, const mguso_bsr& bsr, const mguso_schwarz* sw, RsWork& w, const RsRun& run,
+                 float* x, uint32_t active, float tol, uint32_t max_iter, FusedInst* out, cudaStream_t st) {
   const uint32_t K = run.ninst;
   MG_CHECK_ARG(K >= 1 && K <= PCG_MAX_INST, "resident PCG: 1..8 instances");
   // CTAs per active instance: one each, then one at a time to the instance with the most domains
@@ -1213,6 +1285,17 @@ int pcg_resident(const RsSystem& sys, RsWork& w, const RsRun& run, float* x, uin
     // the vectors of a CTA's vertices, the halo and the hash table have to fit
     const uint64_t need = RS_SCRATCH + 52ull * 32 * dom + 20ull * RS_MAX_HALO + 52ull * dia + 64 + RS_HASH_BYTES;
     if (dom > (uint32_t)RS_MAX_DOM || need > smem) return MGUSO_ERR_UNSUPPORTED;
+    // staged for certain, or looked at row by row (once: more CTAs fit at least as well)
+    const uint32_t stage = 2 * (RS_WARPS / (wide ? 6 : 3)) * RS_CHUNK;
+    if (need - RS_HASH_BYTES + stage <= smem || (w.good[I.k] && I.ncta >= w.good[I.k])) continue;
+    if (I.ncta > w.poor[I.k]) {
+      if (resident_walked(bsr, sw, run, I.k, I.ncta, smem, stage) <= run.walked_max) {
+        w.good[I.k] = I.ncta;
+        continue;
+      }
+      w.poor[I.k] = I.ncta;
+    }
+    return MGUSO_ERR_UNSUPPORTED;
   }
   // records and published sums carry epochs: cleared when allocated and when the epochs run out
   const size_t nrec = 2 * (size_t)std::max<uint32_t>(run.nv, 1), nsum = 3 * (size_t)RS_MAX_G;
@@ -1263,6 +1346,7 @@ int pcg_resident_scene(Scene& s, uint32_t active) {
     r.nv = s.nv;
     r.ninst = K;
     r.nnz = s.Ps.nnz;
+    r.walked_max = WALKED_SCENE;
     for (uint32_t k = 0; k <= K; ++k) r.vert[k] = s.inst_vert[k];
     MG_CHECK_ARG(!sw || resident_domains(*sw, r), "resident PCG: Schwarz domains are not grouped by instance");
     s.rs_ready = true;
@@ -1288,7 +1372,7 @@ int pcg_resident_scene(Scene& s, uint32_t active) {
   MG_TRY(s.fr_inst.reserve(PCG_MAX_INST));
   MG_TRY(s.fr_out.reserve(PCG_MAX_INST));
   // at least one iteration, as the fused kernels run
-  MG_TRY(pcg_resident(y, s.rs, r, s.work.x.p, active, s.p.cg_tol, std::max<uint32_t>(s.p.cg_max_iter, 1), s.fr_inst.p,
+  MG_TRY(pcg_resident(y, *s.A, sw, s.rs, r, s.work.x.p, active, s.p.cg_tol, std::max<uint32_t>(s.p.cg_max_iter, 1), s.fr_inst.p,
                       s.st));
   MG_CUDA(cudaMemcpyAsync(s.fr_out.p, s.fr_inst.p, sizeof(FusedInst) * K, cudaMemcpyDeviceToHost, s.st));
   return MGUSO_OK;

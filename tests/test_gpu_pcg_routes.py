@@ -1,0 +1,40 @@
+"""Which PCG a system is solved by, and that each solves it: the resident one up to where a CTA's rows
+can be kept or staged, the fused kernels (scenes) and the per-kernel PCG (linear-solver seam)
+beyond. mguso_scene_pcg_kernels tells them apart: it names no kernels before a fused solve."""
+import numpy as np
+import pytest
+
+from mguso import CsrMatrix, CudaLinearSolver, ImplicitSolver, scenes
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("precond", ["schwarz", "block"])
+@pytest.mark.parametrize("n", [400, 470, 500])
+def test_solver_around_the_limit(ctx, n, precond):
+    """34, 47 and 53 domains a CTA: rows walked in the BSR, then the per-kernel PCG. The residual formed
+    in float64 against ||b||, bounded as in the resident PCG's tests: 1e-6 by the solver's own FP32
+    recurrence, which drifts by about iterations * 2^-24 (20 to 30 iterations)."""
+    nb, rp, col, val = scenes.grid_bsr(n, seed=n)
+    b = np.random.default_rng(n).standard_normal(3 * nb).astype(np.float32)
+    a = CsrMatrix(*scenes.bsr_to_csr(nb, rp, col, val))
+    for precision in ("mixed", "fp32"):
+        s = CudaLinearSolver(ctx, precond=precond, domain=32, precision=precision)
+        x = s.solve(a, b, 1e-6, 500)
+        st = s.last_stats()
+        assert st.status == 0 and 0 < st.iters < 500
+        assert np.array_equal(x, s.solve(a, b, 1e-6, 500))
+        s.close()
+        r = b.astype(np.float64) - scenes.bsr_spmv_f64(rp, col, val, x)
+        assert np.linalg.norm(r) / np.linalg.norm(b) <= 5e-6
+
+
+@pytest.mark.parametrize("n,precond,fused", [(300, 1, False), (360, 1, True), (330, 2, False), (400, 2, True)])
+def test_scenes_take_the_fused_kernels_where_rows_would_be_walked(ctx, n, precond, fused):
+    """20 and 28 runs a CTA (block Jacobi), 24 and 34 domains (Schwarz)."""
+    sc = scenes.sheet_on_sphere(n, height=0.32)
+    sc["params"] = dict(sc["params"], precond=precond, newton_iters=2)
+    g = ImplicitSolver(ctx, sc, "mixed")
+    assert g.step(1)[0]["status"] == 0
+    assert (g.pcg_kernels() != (-1, -1)) == fused
+    g.close()
