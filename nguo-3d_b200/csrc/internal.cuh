@@ -208,6 +208,7 @@ struct RsSystem {
 struct RsRun {
   int precond = MGUSO_PRECOND_SCHWARZ;
   bool mixed = true, half = false;
+  bool fp64_tiles = false;  // mixed precision: sums over FP16 tiles in FP64 too
   int sms = 148;
   uint32_t nv = 0, ninst = 1;
   uint64_t nnz = 0;  // blocks of A

@@ -1252,8 +1252,10 @@ int pcg_fused_profile(Scene& s, uint32_t iters, float* us2) {
 static int fused_autotune(Scene& s) {
   static std::mutex mu;
   static std::map<std::vector<uint64_t>, std::pair<int, int>> cache;
+  // pcg_mode 2 sums over FP16 tiles in FP64, as only the one-warp domain kernel does
+  const bool fp64_tiles = s.p.pcg_mode == 2 && s.mixed && s.schwarz && s.schwarz->half;
   std::vector<uint64_t> key = {s.nv, s.Ps.nnz, s.ninst, s.mixed ? 1u : 0u,
-                               s.schwarz ? (s.schwarz->half ? 2u : 1u) : 0u, s.schwarz ? s.schwarz->ndom : 0u,
+                               s.schwarz ? (s.schwarz->half ? 2u : 1u) : 0u, s.schwarz ? s.schwarz->ndom : 0u, fp64_tiles,
                                (uint64_t)s.ctx->device};
   {
     std::lock_guard<std::mutex> lock(mu);
@@ -1280,7 +1282,7 @@ static int fused_autotune(Scene& s) {
   s.fr_rows_variant = br;
   int bd = 0;
   if (s.schwarz) {
-    for (int dv = 0; dv < (s.schwarz->half ? N_DOM_VARIANTS : DOM_TC4); ++dv) {
+    for (int dv = 0; dv < (fp64_tiles ? 1 : s.schwarz->half ? N_DOM_VARIANTS : DOM_TC4); ++dv) {
       s.fr_dom_variant = dv;
       MG_TRY(pcg_fused_profile(s, 2, us2));
       MG_TRY(pcg_fused_profile(s, 12, us2));

@@ -37,7 +37,6 @@
 // fixed order that does not depend on timing (where a domain is kept changes no sum), so
 // a solve is reproducible. Data written by other CTAs is read past L1 (ld.cg / volatile).
 #include <algorithm>
-#include <type_traits>
 
 #include "recip.cuh"
 #include "reduce.cuh"
@@ -139,8 +138,9 @@ __device__ __forceinline__ void st_rec(float4* p, float x, float y, float z, uin
 // rows (no bank conflicts, full sectors from L2), every lane multiplies what it holds, and
 // the lanes' partial sums are combined by halving exchanges (a lane keeps half of its sums and
 // gets the partner's for them), 7 shuffles for 32 row sums instead of 32 element loads a lane.
-// Summation type AA: FP32 over FP16 tiles (whose own rounding dwarfs FP32 sums of 32 terms),
-// else the precision's type.
+// Summation type AA: the precision's, but FP32 over FP16 tiles (whose own rounding dwarfs FP32 sums
+// of 32 terms), as the fused three-warp kernels sum, unless the caller asks for FP64 there
+// (pcg_mode 2): two steps of one garment 30.4 -> 32.5 ms, of six 130 -> 147.
 template <class AA, class TS>
 struct TileRegs;
 
@@ -229,6 +229,77 @@ struct TileRegs<AA, __half> {
   }
 };
 
+// FP16 tiles summed in FP64: as above, the FP16 bits moved to where an FP64 number has them (times
+// 2^-1008, exactly, subnormals included; the vectors and the sums take 2^504 each).
+template <>
+struct TileRegs<double, __half> {
+  uint4 u[4];
+  __device__ __forceinline__ void load(const __half* t, int lane) {
+    const uint4* s = reinterpret_cast<const uint4*>(t);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) u[i] = s[32 * i + lane];
+  }
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) u[i] = make_uint4(0, 0, 0, 0);
+  }
+  __device__ __forceinline__ static double lift(double v) { return v * 0x1p504; }
+  __device__ __forceinline__ static uint32_t word(const uint4& v, int t) {
+    return t == 0 ? v.x : t == 1 ? v.y : t == 2 ? v.z : v.w;
+  }
+  __device__ __forceinline__ static double lo(uint32_t w) {
+    return __hiloint2double(((int)(w << 16) >> 6) & (int)0x81fffc00u, 0);
+  }
+  __device__ __forceinline__ static double hi(uint32_t w) {
+    return __hiloint2double(((int)w >> 6) & (int)0x81fffc00u, 0);
+  }
+  __device__ __forceinline__ double rows(const float* __restrict__ v, int lane, int& row) const {
+    const int g = lane >> 2, k = ((lane & 3) ^ (lane >> 3)) & 3;
+    double s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const double c = lift((double)v[8 * i + g]);
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        s[2 * t] = fma(lo(word(u[i], t)), c, s[2 * t]);
+        s[2 * t + 1] = fma(hi(word(u[i], t)), c, s[2 * t + 1]);
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const double send = (g & 4) ? s[t] : s[t + 4], keep = (g & 4) ? s[t + 4] : s[t];
+      s[t] = keep + __shfl_xor_sync(0xffffffffu, send, 18);
+    }
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      const double send = (g & 2) ? s[t] : s[t + 2], keep = (g & 2) ? s[t + 2] : s[t];
+      s[t] = keep + __shfl_xor_sync(0xffffffffu, send, 9);
+    }
+    const double send = (g & 1) ? s[0] : s[1], keep = (g & 1) ? s[1] : s[0];
+    row = 8 * k + g;
+    return lift(keep + __shfl_xor_sync(0xffffffffu, send, 4));
+  }
+  __device__ __forceinline__ double cols(const double* __restrict__ y, int lane, int& col) const {
+    const int g = lane >> 2, k = ((lane & 3) ^ (lane >> 3)) & 3;
+    double z[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const double2 yy = *reinterpret_cast<const double2*>(y + 8 * k + 2 * t);
+      const double y0 = lift(yy.x), y1 = lift(yy.y);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) z[i] = fma(hi(word(u[i], t)), y1, fma(lo(word(u[i], t)), y0, z[i]));
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const double send = (lane & 2) ? z[i] : z[i + 2], keep = (lane & 2) ? z[i + 2] : z[i];
+      z[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
+    }
+    const double send = (lane & 1) ? z[0] : z[1], keep = (lane & 1) ? z[1] : z[0];
+    col = 8 * (lane & 3) + g;
+    return lift(keep + __shfl_xor_sync(0xffffffffu, send, 1));
+  }
+};
+
 // FP32 tiles (element (r, c) at c * 32 + (r ^ c)): lane l holds rows 4w .. 4w + 3, w = l & 7, of
 // the eight columns 4i + h, h = l >> 3; the value at place t of a group is row 4w + (t ^ h).
 template <class AA>
@@ -299,10 +370,9 @@ struct StageNext {
   uint32_t part, tiles, issued;
 };
 
-template <int PRE, class Acc, class TS, int TW>
+template <int PRE, class Acc, class TS, int TW, class AA>
 __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_constant__ RsArgs a) {
   constexpr bool SCH = PRE == MGUSO_PRECOND_SCHWARZ;
-  using AA = typename std::conditional<sizeof(TS) == 2, float, Acc>::type;
   constexpr int TEAMS = RS_WARPS / TW, TEAM = 32 * TW;
   constexpr uint32_t TEAM_BYTES = RS_SCRATCH / TEAMS;  // per-team scratch
   constexpr uint32_t CHUNK_SLOTS = TW == 3 ? 9 : 6;    // whole slots of packed rows per chunk: a multiple of TW
@@ -568,12 +638,16 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
   }
   __syncthreads();
   for (int di = team; di < nD; di += TEAMS) {
-    if (SCH && sizeof(AA) > sizeof(TS) && sizeof(TS) == 4) {
-      // a tile that rs_widen cannot take: its domain's z is NaN, as its product would be
-      const uint32_t n = (uint32_t)(S.fac_off[d0 + di + 1] - S.fac_off[d0 + di]);
-      const float* src = (const float*)S.fac + S.fac_off[d0 + di];
+    if (SCH && sizeof(AA) == 8) {
+      // a tile that has no FP64 image by shifts: its domain's z is NaN, as its product would be
+      const uint32_t n = (uint32_t)((S.fac_off[d0 + di + 1] - S.fac_off[d0 + di]) * sizeof(TS) / 4);
+      const uint32_t* src = (const uint32_t*)((const TS*)S.fac + S.fac_off[d0 + di]);
       bool bad = false;
-      for (uint32_t i = ti; i < n; i += TEAM) bad = bad || !rs_finite(__ldg(src + i));
+      for (uint32_t i = ti; i < n; i += TEAM) {
+        const uint32_t w = __ldg(src + i);
+        bad = bad || (sizeof(TS) == 4 ? (w & 0x7f800000u) == 0x7f800000u
+                                      : (w & 0x7c00u) == 0x7c00u || (w & 0x7c000000u) == 0x7c000000u);
+      }
       if (bad) s_scale[di] = __uint_as_float(0x7fffffffu);
     }
     if (s_tofs[di] == RS_EMPTY) continue;
@@ -930,7 +1004,8 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
         else
           t.zero();
       };
-      if (SCH && sizeof(TS) == 2) {  // in registers for both passes
+      constexpr bool KEEP = sizeof(TS) == 2 && sizeof(AA) == 4;  // in registers for both passes
+      if (SCH && KEEP) {
         load(ta, q);
         if (TW == 3) load(tb, q + 3);
       }
@@ -949,15 +1024,15 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
       }
       if (TW == 3 || ti < 96) rd[ti] = r;
       team_sync(team);
-      if (staged) stage_issue();  // the tiles are in registers
+      if (KEEP && staged) stage_issue();  // the tiles are in registers
       float zi = 0.f;
       if (SCH) {
         int at;
-        if (sizeof(TS) == 4) load(ta, q);
+        if (!KEEP) load(ta, q);
         AA v = ta.rows(rd + 32 * rs_tile_j(q), lane, at);
         AA v2 = 0;
         if (TW == 3) {
-          if (sizeof(TS) == 4) load(tb, q + 3);
+          if (!KEEP) load(tb, q + 3);
           v2 = tb.rows(rd + 32 * rs_tile_j(q + 3), lane, at);
         }
         part[32 * q + at] = v;
@@ -971,15 +1046,16 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
           yd[ti] = y;
         }
         team_sync(team);
-        if (sizeof(TS) == 4 && (TW == 3 || sizeof(AA) == 8)) load(ta, q);
+        if (!KEEP && (TW == 3 || sizeof(AA) == 8)) load(ta, q);
         v = ta.cols(yd + 32 * rs_tile_i(q), lane, at);
         if (TW == 3) {
-          if (sizeof(TS) == 4) load(tb, q + 3);
+          if (!KEEP) load(tb, q + 3);
           v2 = tb.cols(yd + 32 * rs_tile_i(q + 3), lane, at);
         }
         part[32 * q + at] = v;
         if (TW == 3) part[32 * (q + 3) + at] = v2;
         team_sync(team);
+        if (!KEEP && staged) stage_issue();
         if (TW == 3 || q < 3) {  // z of tile column q
           AA z = part[32 * (q * (q + 1) / 2 + q) + lane];
           if (q < 2) z += part[32 * ((q + 1) * (q + 2) / 2 + q) + lane];
@@ -1192,13 +1268,16 @@ static uint32_t resident_walked(const mguso_bsr& a, const mguso_schwarz* sw, con
   return worst;
 }
 
+template <class Acc, class TS, int TW, class AA = Acc>
+static void* schwarz_kernel() {
+  return (void*)k_pcg_resident<MGUSO_PRECOND_SCHWARZ, Acc, TS, TW, AA>;
+}
+
 template <int TW>
-static void* resident_kernel(bool mixed, bool half) {
-  if (half)
-    return mixed ? (void*)k_pcg_resident<MGUSO_PRECOND_SCHWARZ, double, __half, TW>
-                 : (void*)k_pcg_resident<MGUSO_PRECOND_SCHWARZ, float, __half, TW>;
-  return mixed ? (void*)k_pcg_resident<MGUSO_PRECOND_SCHWARZ, double, float, TW>
-               : (void*)k_pcg_resident<MGUSO_PRECOND_SCHWARZ, float, float, TW>;
+static void* resident_kernel(const RsRun& run) {
+  if (!run.half) return run.mixed ? schwarz_kernel<double, float, TW>() : schwarz_kernel<float, float, TW>();
+  if (!run.mixed) return schwarz_kernel<float, __half, TW>();
+  return run.fp64_tiles ? schwarz_kernel<double, __half, TW>() : schwarz_kernel<double, __half, TW, float>();
 }
 
 int pcg_resident(const RsSystem& sys, const mguso_bsr& bsr, const mguso_schwarz* sw, RsWork& w, const RsRun& run,
@@ -1258,10 +1337,10 @@ int pcg_resident(const RsSystem& sys, const mguso_bsr& bsr, const mguso_schwarz*
   // turns. Block Jacobi has no tiles to share and loses (100 x 100: 2.70 -> 2.76).
   const int wide = run.precond == MGUSO_PRECOND_SCHWARZ && most <= 3 ? 1 : 0;
   void* fn = run.precond == MGUSO_PRECOND_BLOCK_JACOBI
-                 ? (run.mixed ? (void*)k_pcg_resident<MGUSO_PRECOND_BLOCK_JACOBI, double, float, 3>
-                              : (void*)k_pcg_resident<MGUSO_PRECOND_BLOCK_JACOBI, float, float, 3>)
-             : wide ? resident_kernel<6>(run.mixed, run.half)
-                    : resident_kernel<3>(run.mixed, run.half);
+                 ? (run.mixed ? (void*)k_pcg_resident<MGUSO_PRECOND_BLOCK_JACOBI, double, float, 3, double>
+                              : (void*)k_pcg_resident<MGUSO_PRECOND_BLOCK_JACOBI, float, float, 3, float>)
+             : wide ? resident_kernel<6>(run)
+                    : resident_kernel<3>(run);
   if (w.fn[wide] != fn) {
     w.fn[wide] = nullptr;
     w.smem[wide] = 0;
@@ -1342,6 +1421,7 @@ int pcg_resident_scene(Scene& s, uint32_t active) {
     r.precond = sw ? MGUSO_PRECOND_SCHWARZ : MGUSO_PRECOND_BLOCK_JACOBI;
     r.mixed = s.mixed;
     r.half = sw && sw->half;
+    r.fp64_tiles = s.p.pcg_mode == 2;
     r.sms = s.ctx->sm_count;
     r.nv = s.nv;
     r.ninst = K;

@@ -38,3 +38,23 @@ def test_scenes_take_the_fused_kernels_where_rows_would_be_walked(ctx, n, precon
     assert g.step(1)[0]["status"] == 0
     assert (g.pcg_kernels() != (-1, -1)) == fused
     g.close()
+
+
+@pytest.mark.parametrize("n", [40, 130, 330, 400])
+def test_mode_2_sums_over_fp16_tiles_in_fp64(ctx, n):
+    """Mixed precision with FP16 tiles and pcg_mode 2: one, four and 24 (staged) domains a CTA and the fused
+    kernels. Against the fused pair whose one-warp domain kernel sums in FP64 (pcg_variant 1), after
+    four iterations from a rough right-hand side that moves vertices by a metre: FP64 sums in another
+    order differ by 1e-13 or less of their terms, so a result rounds to another FP32 number for one entry in
+    1e5 at most, where FP32 sums (1e-7) change every third to fiftieth."""
+    sc = scenes.sheet_on_sphere(n, height=2.0)
+    sc["velocities"] = (60 * np.random.default_rng(n).standard_normal(sc["positions"].shape)).astype(np.float32)
+    out = []
+    for kw in (dict(pcg_variant=1), dict(pcg_mode=2)):
+        p = dict(sc["params"], self_collision=0, newton_iters=1, cg_max_iter=4, cg_tol=1e-9, **kw)
+        g = ImplicitSolver(ctx, dict(sc, params=p), "mixed")
+        assert g.step(1)[0]["status"] == 0
+        out.append(g.positions.copy())
+        g.close()
+    assert np.abs(out[0] - sc["positions"]).max() > 0.5
+    assert (out[0] == out[1]).mean() >= 0.999
