@@ -32,10 +32,12 @@
 // block of a row, for the preconditioner every third tile. Where a CTA has three domains or
 // fewer, six warps do (36 warps in six such teams were no faster: 64 registers a thread spill).
 //
-// The CTAs are resident together (cooperative launch). Every poll is bounded: a CTA that gives
-// up sets its instance's status and leaves, and the others follow. Dot products are summed in a
+// The CTAs are resident together (cooperative launch), so a solve takes the whole chip and starts
+// once other kernels leave it to it (20 s of another stream's kernel delayed a solve by 20 s).
+// Every poll is bounded: a CTA that gives up sets its instance's status and leaves, and the
+// others follow. Dot products are summed in a
 // fixed order that does not depend on timing (where a domain is kept changes no sum), so
-// a solve is reproducible. Data written by other CTAs is read past L1 (ld.cg / volatile).
+// a solve is reproducible. Data written by other CTAs is read past L1 (relaxed loads of 16 bytes).
 #include <algorithm>
 
 #include "recip.cuh"
@@ -58,6 +60,12 @@ constexpr uint32_t RS_EMPTY = 0xffffffffu;
 constexpr uint32_t RS_WIDE = 8;  // rows that make a slot worth padding to 32
 constexpr uint32_t RS_ALWAYS = 0xffffffffu;  // epoch of a record that holds for the whole solve
 constexpr int RS_MAX_G = 160;
+// An exchange waits for the slowest CTA's phase: up to seconds. A record was stored before the exchange
+// that its reader has passed, so only the store's way to L2 is waited for (a microsecond or two;
+// 10 ms at most). That limit is each record's own, so a CTA that misses several (3 of a halo, or
+// those of a row walked in the BSR) takes that many: a look at s_abort in the poll, inlined or
+// not, cost the iterations registers (two steps of one garment 37.7 -> 38.3 to 39.5 ms).
+constexpr uint32_t RS_EXCHANGE_POLLS = 1u << 22, RS_RECORD_POLLS = 1u << 14;
 
 struct RsInst {
   uint32_t k, cta0, ncta;
@@ -764,7 +772,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
         for (uint32_t tries = 0;; ++tries) {
           asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(count) : "memory");
           if ((int)(seen - target) >= 0) break;
-          if (tries > (1u << 22)) {  // gives up after seconds
+          if (tries > RS_EXCHANGE_POLLS) {
             ok = false;
             break;
           }
@@ -822,7 +830,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pcg_resident(const __grid_con
       z = ld_rlx(a.rec + 2 * pos);
       p = ld_rlx(a.rec + 2 * pos + 1);
       if ((z.w == epoch || z.w == RS_ALWAYS) && (p.w == epoch || p.w == RS_ALWAYS)) break;
-      if (tries > (1u << 22)) {
+      if (tries > RS_RECORD_POLLS) {
         atomicOr(&a.out[I.k].status, ST_WAIT_TIMEOUT);
         s_abort = 1;
         break;
