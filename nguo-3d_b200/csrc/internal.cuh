@@ -236,9 +236,9 @@ struct RsWork {
 
 // Solves the instances of `active` into x (3 floats per vertex; the others get x = 0) and
 // their results into out[k] (device), enqueued on st without a host wait. Returns
-// MGUSO_ERR_UNSUPPORTED, having enqueued nothing, when the system's vectors do not fit in the
-// SMs' shared memory (beyond about 64 domains or 2 000 vertices per SM) or too many of its blocks
-// have no place beside them. a, sw: its pattern and domains on the host (sw null: block Jacobi).
+// MGUSO_ERR_UNSUPPORTED, having solved nothing, when the system's vectors do not fit in the SMs'
+// shared memory (beyond about 64 domains or 2 000 vertices per SM), too many of its blocks have no
+// place beside them, or the device refuses a grid of all its SMs. a, sw: its pattern and domains on the host (sw null: block Jacobi).
 int pcg_resident(const RsSystem& sys, const mguso_bsr& a, const mguso_schwarz* sw, RsWork& w, const RsRun& run,
                  float* x, uint32_t active, float tol, uint32_t max_iter, FusedInst* out, cudaStream_t st);
 

@@ -40,6 +40,7 @@
 // a solve is reproducible. Data written by other CTAs is read past L1 (relaxed loads of 16 bytes).
 #include <algorithm>
 
+#include "coop.cuh"
 #include "recip.cuh"
 #include "reduce.cuh"
 #include "scene.cuh"
@@ -1417,7 +1418,13 @@ int pcg_resident(const RsSystem& sys, const mguso_bsr& bsr, const mguso_schwarz*
   k_rs_reset<<<64, 256, 0, st>>>(a.count, out, K, x, 3 * run.nv);
   MG_CUDA(cudaGetLastError());
   void* args[] = {(void*)&a};
-  MG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(RS_THREADS), args, smem, st));
+  const cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(RS_THREADS), args, smem, st);
+  if (coop_refused(e)) {
+    cudaGetLastError();
+    w.smem[wide] = 0;  // nor will it be the next time
+    return MGUSO_ERR_UNSUPPORTED;
+  }
+  MG_CUDA(e);
   return MGUSO_OK;
 }
 
