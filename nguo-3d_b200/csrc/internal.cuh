@@ -212,13 +212,15 @@ struct RsRun {
   int sms = 148;
   uint32_t nv = 0, ninst = 1;
   uint64_t nnz = 0;  // blocks of A
-  // of a CTA's blocks, how many in a thousand may have no place packed before the solve is left to
-  // the other PCG (resident_walked)
+  // how many of a CTA's blocks may have no place packed before the solve is left to the other PCG
+  // (resident_walked)
   uint32_t walked_max = 0;
   uint32_t vert[PCG_MAX_INST + 1] = {}, dom[PCG_MAX_INST + 1] = {}, diag[PCG_MAX_INST] = {};
 };
 
-constexpr uint32_t WALKED_SCENE = 100, WALKED_SOLVER = 780;  // walked_max: see resident_walked
+// walked_max: see resident_walked
+constexpr uint32_t WALKED_SCENE = 1500;
+inline uint32_t walked_solver(bool schwarz, uint32_t nv) { return schwarz ? 2800 + nv / 42 : 12000; }
 
 struct RsWork {
   // per team size: the kernel that `smem` was found for and its dynamic shared memory (0: it cannot

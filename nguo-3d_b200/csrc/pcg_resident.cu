@@ -1205,21 +1205,22 @@ bool resident_domains(const mguso_schwarz& s, RsRun& run) {
   return d == s.ndom;
 }
 
-// Of the blocks of one CTA, the largest share (in thousandths, over instance k's CTAs) that would be
-// walked in the BSR because their rows are neither resident nor staged, found as the kernel's set-up
-// places them (without contact blocks, which only the device knows, and isolated vertices, which
-// bear no load in a scene). A walked block costs two polled records, so a chip full of them
-// loses to the other PCGs. us an iteration, walked there or not -> with the other PCG:
-//   scenes, Schwarz, mixed: 300 x 300 sheet (20 domains a CTA, all staged) 24 -> 37; six garments (29,
-//     staged) 31 -> 53; seven (31, the worst CTA walks 78%) 88 -> 60; eight (37, 85%) 102 -> 73;
-//   scenes, block Jacobi: 300 x 300 sheet (20, staged) 20 -> 27; 360 x 360 (28, 79%) 39 -> 29; five
-//     garments (33, 80%) 42 -> 29; 545 x 545 sheet 134 -> 53;
-//   solver, Schwarz, mixed (7 blocks a row): 360 x 360 grid (28, 0%) 45 -> 74; 400 x 400 (34, 65%) 74 -> 84;
-//     440 (41, 76%) 93 -> 95; 460 (45, 80%) 103 -> 99; 480 112 -> 103;
-//   solver, Schwarz, FP32: 400 68 -> 74; 440 87 -> 86; 460 92 -> 84;
-//   solver, block Jacobi, mixed: 460 (45, 78%) 32 -> 35; 480 (49, 82%) 38 -> 38; 545 61 -> 49.
-// The share jumps where the staging buffers (147 KB) no longer fit beside a CTA's vectors. So
-// scenes allow a tenth (WALKED_SCENE), the solver, whose other PCG takes five launches, 78%.
+// The most blocks that one of instance k's CTAs would walk in the BSR, because their rows are neither
+// resident nor staged or its halo outgrows the table; found as the kernel's set-up places rows
+// (without contact blocks, which only the device knows, and isolated vertices, which bear no load in
+// a scene). A walked block costs two polled records, 4 ns of its CTA's time, for which the others
+// wait, so a chip full of them loses to the other PCGs. us an iteration, resident and the other
+// (in brackets: thousands of blocks walked by the worst CTA):
+//   scenes, Schwarz, mixed: 300 x 300 sheet (0) 24, 37; six garments (0) 31, 53; seven (11) 88, 60; eight 102, 73;
+//   scenes, block Jacobi: 300 x 300 sheet (0) 20, 27; 360 x 360 (9) 39, 29; five garments 42, 29; 545 x
+//     545 sheet 134, 53;
+//   solver, Schwarz, mixed: 360 x 360 grid (7 blocks a row; 0) 51, 78; 400 x 400 (4.9) 81, 89; 440 (6.9) 102,
+//     102; 480 (9.1) 121, 116; 330 x 330 with 13 blocks a row (0) 48, 76, 360 (8.9) 95, 88; 20 thousand
+//     vertices with 8 random neighbours each (3.7, halo of 3 300) 44, 40, 40 thousand (7.5) 82, 52;
+//   solver, block Jacobi, mixed: 400 (4.9) 26, 40; 480 (8.9) 38, 47; 520 (11) 46, 56; with 13 blocks a row
+//     400 (12) 53, 54, 440 (15) 74, 65; 90 thousand vertices with random neighbours (5.5) 38, 44.
+// So scenes, whose other PCG takes two launches an iteration, allow WALKED_SCENE blocks; the solver, whose
+// other takes four over vectors in memory, walked_solver.
 static uint32_t resident_walked(const mguso_bsr& a, const mguso_schwarz* sw, const RsRun& run, uint32_t k,
                                 uint32_t ncta, uint32_t smem, uint32_t stage) {
   const uint32_t v0 = run.vert[k], nv = run.vert[k + 1] - v0;
@@ -1272,7 +1273,7 @@ static uint32_t resident_walked(const mguso_bsr& a, const mguso_schwarz* sw, con
       else if (!(m.blocks < 60000u && staged && m.tail <= RS_CHUNK))
         walked += m.blocks;
     }
-    worst = std::max(worst, (uint32_t)(1000 * walked / std::max<uint64_t>(blocks, 1)));
+    worst = std::max(worst, (uint32_t)(halo > RS_MAX_HALO ? blocks : walked));
   }
   return worst;
 }
@@ -1373,9 +1374,9 @@ int pcg_resident(const RsSystem& sys, const mguso_bsr& bsr, const mguso_schwarz*
     // the vectors of a CTA's vertices, the halo and the hash table have to fit
     const uint64_t need = RS_SCRATCH + 52ull * 32 * dom + 20ull * RS_MAX_HALO + 52ull * dia + 64 + RS_HASH_BYTES;
     if (dom > (uint32_t)RS_MAX_DOM || need > smem) return MGUSO_ERR_UNSUPPORTED;
-    // staged for certain, or looked at row by row (once: more CTAs fit at least as well)
+    // looked at row by row, once: more CTAs fit at least as well
     const uint32_t stage = 2 * (RS_WARPS / (wide ? 6 : 3)) * RS_CHUNK;
-    if (need - RS_HASH_BYTES + stage <= smem || (w.good[I.k] && I.ncta >= w.good[I.k])) continue;
+    if (w.good[I.k] && I.ncta >= w.good[I.k]) continue;
     if (I.ncta > w.poor[I.k]) {
       if (resident_walked(bsr, sw, run, I.k, I.ncta, smem, stage) <= run.walked_max) {
         w.good[I.k] = I.ncta;

@@ -12,8 +12,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("precond", ["schwarz", "block"])
 @pytest.mark.parametrize("n", [400, 470, 500])
 def test_solver_around_the_limit(ctx, n, precond):
-    """34, 47 and 53 domains a CTA: rows walked in the BSR, then the per-kernel PCG. The residual formed
-    in float64 against ||b||, bounded as in the resident PCG's tests: 1e-6 by the solver's own FP32
+    """34, 47 and 53 domains a CTA: rows walked in the BSR, with Schwarz from 47 on the per-kernel PCG. The
+    residual formed in float64 against ||b||, bounded as in the resident PCG's tests: 1e-6 by the solver's own FP32
     recurrence, which drifts by about iterations * 2^-24 (20 to 30 iterations)."""
     nb, rp, col, val = scenes.grid_bsr(n, seed=n)
     b = np.random.default_rng(n).standard_normal(3 * nb).astype(np.float32)
@@ -58,3 +58,36 @@ def test_mode_2_sums_over_fp16_tiles_in_fp64(ctx, n):
         g.close()
     assert np.abs(out[0] - sc["positions"]).max() > 0.5
     assert (out[0] == out[1]).mean() >= 0.999
+
+
+@pytest.mark.parametrize("nv", [5000, 20000, 60000])
+def test_random_patterns(ctx, nv):
+    """Eight random neighbours a vertex: halos of up to ten thousand vertices a CTA, past the resident
+    table's 1 536, and Schwarz domains of one to 32 vertices. Diagonally dominant, so 20 to 30 iterations;
+    residual in float64 and its bound as above."""
+    rng = np.random.default_rng(nv)
+    e = rng.integers(0, nv, (4 * nv, 2))
+    e = np.unique(np.sort(e[e[:, 0] != e[:, 1]], 1), axis=0)
+    d = rng.standard_normal((len(e), 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    blk = d[:, :, None] * d[:, None, :]
+    diag = np.tile(2.0 * np.eye(3), (nv, 1, 1))
+    np.add.at(diag, e[:, 0], blk)
+    np.add.at(diag, e[:, 1], blk)
+    rows = np.concatenate([np.arange(nv), e[:, 0], e[:, 1]])
+    cols = np.concatenate([np.arange(nv), e[:, 1], e[:, 0]])
+    vals = np.concatenate([diag, -blk, -blk]).astype(np.float32)
+    o = np.lexsort((cols, rows))
+    rp = np.zeros(nv + 1, np.int64)
+    np.cumsum(np.bincount(rows, minlength=nv), out=rp[1:])
+    rp, cols, vals = rp.astype(np.uint32), cols[o].astype(np.uint32), vals[o]
+    b = rng.standard_normal(3 * nv).astype(np.float32)
+    a = CsrMatrix(*scenes.bsr_to_csr(nv, rp, cols, vals))
+    for precond in ("schwarz", "block"):
+        s = CudaLinearSolver(ctx, precond=precond, domain=32)
+        x = s.solve(a, b, 1e-6, 500)
+        st = s.last_stats()
+        assert st.status == 0 and 0 < st.iters < 500
+        s.close()
+        r = b.astype(np.float64) - scenes.bsr_spmv_f64(rp, cols, vals, x)
+        assert np.linalg.norm(r) / np.linalg.norm(b) <= 5e-6
