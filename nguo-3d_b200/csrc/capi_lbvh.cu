@@ -1,5 +1,4 @@
 // extern "C" entry points of the LBVH broad phase and the radix sort.
-#include <cmath>
 #include <cstring>
 
 #include "lbvh.cuh"
@@ -58,28 +57,7 @@ int mguso_lbvh_download(mguso_lbvh* b, uint64_t* keys, uint32_t* perm, uint32_t*
     }
   }
   if (perm && nt) MG_CUDA(cudaMemcpy(perm, L.perm.p, 4 * (size_t)nt, cudaMemcpyDeviceToHost));
-  if (nt > 1 && (left || right || node_boxes)) {
-    // the children's indices and the node's box (their union) from its record
-    std::vector<float4> r(4 * (size_t)(nt - 1));
-    MG_CUDA(cudaMemcpy(r.data(), L.rec.p, sizeof(float4) * r.size(), cudaMemcpyDeviceToHost));
-    // as the refit's minima: a NaN gives way, -0 is below +0
-    auto least = [](float u, float v) { return u == v ? (std::signbit(u) ? u : v) : std::fmin(u, v); };
-    auto most = [](float u, float v) { return u == v ? (std::signbit(u) ? v : u) : std::fmax(u, v); };
-    for (uint32_t i = 0; i + 1 < nt; ++i) {
-      const float4 *a = &r[4 * (size_t)i], *b = a + 2;
-      if (left) std::memcpy(left + i, &a[0].w, 4);
-      if (right) std::memcpy(right + i, &b[0].w, 4);
-      if (node_boxes) {
-        float* o = node_boxes + 6 * (size_t)i;
-        o[0] = least(a[0].x, b[0].x);
-        o[1] = least(a[0].y, b[0].y);
-        o[2] = least(a[0].z, b[0].z);
-        o[3] = most(a[1].x, b[1].x);
-        o[4] = most(a[1].y, b[1].y);
-        o[5] = most(a[1].z, b[1].z);
-      }
-    }
-  }
+  if (nt > 1 && (left || right || node_boxes)) MG_TRY(lbvh_nodes(&L, left, right, node_boxes));
   return MGUSO_OK;
 }
 

@@ -709,6 +709,39 @@ int lbvh_refit_pos(Lbvh* b, const float* pos, const uint32_t* tris, cudaStream_t
   return b->nt ? launch_refit(b, pos, tris, b->rec.p, s) : MGUSO_OK;
 }
 
+// A node's children and its box, the union of its record's two halves (taken as the refit takes it).
+__global__ void k_nodes(const float4* __restrict__ rec, uint32_t n, uint32_t* __restrict__ left,
+                        uint32_t* __restrict__ right, float* __restrict__ boxes) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float4* r = rec + 4 * (size_t)i;
+  const float4 l0 = r[0], h0 = r[1], l1 = r[2], h1 = r[3];
+  left[i] = __float_as_uint(l0.w);
+  right[i] = __float_as_uint(l1.w);
+  float* o = boxes + 6 * (size_t)i;
+  o[0] = fminf(l0.x, l1.x);
+  o[1] = fminf(l0.y, l1.y);
+  o[2] = fminf(l0.z, l1.z);
+  o[3] = fmaxf(h0.x, h1.x);
+  o[4] = fmaxf(h0.y, h1.y);
+  o[5] = fmaxf(h0.z, h1.z);
+}
+
+int lbvh_nodes(Lbvh* b, uint32_t* left, uint32_t* right, float* boxes) {
+  const uint32_t n = b->nt - 1;
+  cudaStream_t s = b->ctx->stream;
+  MG_TRY(b->nodes.reserve(8 * (size_t)n));
+  uint32_t *dl = b->nodes.p, *dr = dl + n;
+  float* db = reinterpret_cast<float*>(dr + n);
+  k_nodes<<<ceil_div(n, 256), 256, 0, s>>>(b->rec.p, n, dl, dr, db);
+  MG_CUDA(cudaGetLastError());
+  if (left) MG_CUDA(cudaMemcpyAsync(left, dl, 4 * (size_t)n, cudaMemcpyDeviceToHost, s));
+  if (right) MG_CUDA(cudaMemcpyAsync(right, dr, 4 * (size_t)n, cudaMemcpyDeviceToHost, s));
+  if (boxes) MG_CUDA(cudaMemcpyAsync(boxes, db, 24 * (size_t)n, cudaMemcpyDeviceToHost, s));
+  MG_CUDA(cudaStreamSynchronize(s));
+  return MGUSO_OK;
+}
+
 int lbvh_build(Lbvh* b, const float* pos, uint32_t nv, const uint32_t* tris, uint32_t nt, int key_bits,
                cudaStream_t s) {
   (void)nv;

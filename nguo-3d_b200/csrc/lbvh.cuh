@@ -37,6 +37,7 @@ struct Lbvh {
   DevBuf<unsigned char> rs_tmpk;
   // query scratch
   DevBuf<uint32_t> qkeys, qorder;
+  DevBuf<uint32_t> nodes;  // of lbvh_nodes: 8 words per inner node
   // optional per-stage timing events: 0 start, 1 morton, 2 sort, 3 karras, 4 refit,
   // 5 query prep, 6 traversal
   bool ev_on = false;
@@ -54,6 +55,9 @@ int lbvh_refit_pos(Lbvh* b, const float* pos, const uint32_t* tris, cudaStream_t
 // The displacement records (AABB of dx over each primitive's vertices, refitted up the tree), for
 // the CCD's pruning test.
 int lbvh_refit_disp(Lbvh* b, const float* dx, const uint32_t* tris, cudaStream_t s);
+// The nodes as the caller of a build sees them: children and boxes (lo, hi) of each, to host memory
+// (null: not wanted), once every stream has passed the build.
+int lbvh_nodes(Lbvh* b, uint32_t* left, uint32_t* right, float* boxes);
 int lbvh_query_points(Lbvh* b, const float* pts, uint32_t np, float dhat, uint32_t* pairs, uint64_t cap,
                       unsigned long long* count, bool morton_order, cudaStream_t s);
 
