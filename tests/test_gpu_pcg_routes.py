@@ -91,3 +91,32 @@ def test_random_patterns(ctx, nv):
         s.close()
         r = b.astype(np.float64) - scenes.bsr_spmv_f64(rp, cols, vals, x)
         assert np.linalg.norm(r) / np.linalg.norm(b) <= 5e-6
+
+
+def test_solvers_on_threads_share_the_gpu():
+    """Three threads, each with its own context and solver, solve at once: every launch wants all SMs, so
+    they take turns, and each solution is the one a solver alone finds, bit for bit."""
+    import threading
+
+    from mguso import Context
+
+    nb, rp, col, val = scenes.grid_bsr(100, seed=2)  # more domains than SMs
+    a = CsrMatrix(*scenes.bsr_to_csr(nb, rp, col, val))
+    b = np.random.default_rng(1).standard_normal(3 * nb).astype(np.float32)
+    out = [[], [], []]
+
+    def work(mine):
+        ctx = Context(0)
+        s = CudaLinearSolver(ctx, precond="schwarz", domain=32)
+        for _ in range(20):
+            mine.append(s.solve(a, b, 1e-6, 500))
+        s.close()
+        ctx.close()
+
+    threads = [threading.Thread(target=work, args=(mine,)) for mine in out]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert [len(mine) for mine in out] == [20, 20, 20]
+    assert all(np.array_equal(x, out[0][0]) for mine in out for x in mine)
