@@ -608,8 +608,8 @@ def run_batch(args, dist: Dist):
         "higher_is_better": True,
         "scaling": "weak",
         "vs_baseline": None,
-        "dtype": "f32 storage + f64 (dots, norms, SpMV/apply accumulation, barrier, CCD root); "
-                 "Schwarz factor tiles f16 scaled per domain",
+        "dtype": "f32 storage + f64 (dots, norms, SpMV accumulation, barrier, CCD root); "
+                 "Schwarz factor tiles f16 scaled per domain, summed in f32",
         "data": "synthetic (seeded meshes; no dataset)",
         "config": {
             "workload": BATCH_WORKLOAD,

@@ -29,7 +29,7 @@ extern "C" {
 #define MGUSO_ERR_PCG_CAP 4       /* PCG hit max_iter before reaching tol */
 #define MGUSO_ERR_CCD_CAP 5       /* a CCD root solve hit its iteration cap */
 #define MGUSO_ERR_PAIR_OVERFLOW 6 /* candidate-pair buffer too small (count still reported) */
-#define MGUSO_ERR_BVH_STACK 7     /* LBVH traversal stack overflow */
+#define MGUSO_ERR_BVH_STACK 7     /* an LBVH walk's node queue overflowed */
 #define MGUSO_ERR_CUDA 8          /* a CUDA runtime call failed */
 #define MGUSO_ERR_TIMEOUT 9       /* a bounded device wait gave up */
 #define MGUSO_ERR_UNSUPPORTED 10  /* configuration not supported */
@@ -93,7 +93,14 @@ int mguso_linear_solver_destroy(mguso_linear_solver* s);
 /* solve(a, b, tol, max_iter) -> x  (LinearSolver::solve). a, b, x host; x has a->n
  * entries. Stats as LinearSolver::last_stats. Reaching max_iter is reported in
  * stats->status; the return value is still MGUSO_OK and x holds the last iterate, as in
- * the reference, which returns the best x without failing. */
+ * the reference, which returns the best x without failing.
+ *
+ * One-level solves (here and in mguso_step, pcg_mode 0 and 2) run as one cooperative launch of a
+ * thread block on every SM, so they start once the kernels of other streams have left the GPU to
+ * them and hold all of it meanwhile. Its blocks wait for one another with bounded polls: one that
+ * gives up (seconds) ends the call, or the step, with MGUSO_ERR_TIMEOUT. Where the process may not
+ * use all SMs, or the system does not fit on them, the kernels of pcg_mode 1 (in a step, the fused
+ * kernels) solve it. */
 int mguso_linear_solve(mguso_linear_solver* s, const mguso_csr* a, const float* b, float tol,
                        uint32_t max_iter, float* x, mguso_lin_stats* stats);
 

@@ -72,7 +72,7 @@ int mguso_lbvh_status(mguso_lbvh* b) {
     return MGUSO_ERR_TIMEOUT;
   }
   if (st & ST_STACK_OVERFLOW) {
-    set_error("LBVH traversal stack overflow (64 entries)");
+    set_error("LBVH point walk: a node queue overflowed");
     return MGUSO_ERR_BVH_STACK;
   }
   if (st & ST_PAIR_OVERFLOW) {

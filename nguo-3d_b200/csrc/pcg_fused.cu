@@ -1181,7 +1181,7 @@ int pcg_fused_results(Scene& s, uint32_t K, PcgInstResult* out) {
     out[k].status = hi[k].status;
     out[k].done = hi[k].done;
     if (hi[k].status & ST_WAIT_TIMEOUT) {
-      set_error("fused PCG: a bounded bulk-copy wait timed out");
+      set_error("PCG: a bounded wait between thread blocks or for a bulk copy timed out");
       return MGUSO_ERR_TIMEOUT;
     }
   }

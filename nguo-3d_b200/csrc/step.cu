@@ -146,8 +146,8 @@ static int linear_solve(Scene& s, uint32_t active, mguso_lin_stats* ls, bool* de
   const bool two_level = s.schwarz && s.schwarz->levels == 2;
   if (!two_level && (s.p.pcg_mode == 0 || s.p.pcg_mode == 2 || s.ninst > 1)) {
     // the resident kernel, unless the caller fixes a pair of fused kernels or the system is too
-    // large for it (two steps of six garments 115 ms against 179 ms with the fused kernels, of one
-    // garment 38 against 74, a 64 x 64 sheet's step 9.0 against 16.3)
+    // large for it (us an iteration, resident and fused: a 64 x 64 sheet 6 and 17, one garment 9.5
+    // and 25, six 31 and 53; where it ends: resident_walked)
     int rc = s.p.pcg_variant > 0 ? MGUSO_ERR_UNSUPPORTED : pcg_resident_scene(s, active);
     if (rc == MGUSO_ERR_UNSUPPORTED) {
       MG_TRY(pcg_fused_select(s));

@@ -289,13 +289,13 @@ class ImplicitSolver:
         return out
 
     def pcg_kernels(self) -> tuple:
-        """(rows variant, domain variant) of the fused PCG in use (-1 before the first solve)."""
+        """(rows variant, domain variant) of the fused PCG (-1 before the first fused solve or profile)."""
         out = np.zeros(2, np.int32)
         check(self.lib.mguso_scene_pcg_kernels(self.h, ptr(out)))
         return int(out[0]), int(out[1])
 
     def pcg_kernel_names(self) -> dict:
-        """Kernel names of the fused PCG in use, for the mixed-precision FP16-tile step."""
+        """Kernel names of the fused PCG, for the mixed-precision FP16-tile step."""
         rv, dv = self.pcg_kernels()
         rows = "k_fr_rows_sell<double>" if rv == 3 else f"k_fr_rows<double, {({0: 2, 1: 1, 2: 4}).get(rv, 2)}>"
         if dv >= 4:
