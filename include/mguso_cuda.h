@@ -251,8 +251,9 @@ typedef struct {
                                  or with block Jacobi 650 vertices, per SM) and scenes with a
                                  pcg_variant run two fused kernels per iteration (rows, domains)
                                  at full occupancy, replayed as CUDA graphs. Over FP16 factor
-                                 tiles mixed precision sums in FP32 in mode 0 (in FP64 with the
-                                 one-warp domain kernel of a pcg_variant) and in FP64 in mode 2;
+                                 tiles mixed precision sums in FP32 in mode 0 (in FP64 for Schwarz
+                                 domains of 10 vertices or fewer and with the one-warp domain
+                                 kernel of a pcg_variant) and in FP64 in mode 2;
                               1: one launch per PCG kernel, replayed as CUDA graphs (single
                                  scenes only) */
   int factor_storage;      /* Schwarz factor tiles: 0 = by precision (FP32 tiles with

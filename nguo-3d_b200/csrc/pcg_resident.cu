@@ -149,7 +149,8 @@ __device__ __forceinline__ void st_rec(float4* p, float x, float y, float z, uin
 // gets the partner's for them), 7 shuffles for 32 row sums instead of 32 element loads a lane.
 // Summation type AA: the precision's, but FP32 over FP16 tiles (whose own rounding dwarfs FP32 sums
 // of 32 terms), as the fused three-warp kernels sum, unless the caller asks for FP64 there
-// (pcg_mode 2): two steps of one garment 30.4 -> 32.5 ms, of six 130 -> 147.
+// (pcg_mode 2): two steps of one garment 30.4 -> 32.5 ms, of six 130 -> 147. Domains of one tile (10
+// vertices or fewer), for which the one-warp kernel is the faster of the fused ones, take its FP64 sums.
 template <class AA, class TS>
 struct TileRegs;
 
@@ -1437,7 +1438,7 @@ int pcg_resident_scene(Scene& s, uint32_t active) {
     r.precond = sw ? MGUSO_PRECOND_SCHWARZ : MGUSO_PRECOND_BLOCK_JACOBI;
     r.mixed = s.mixed;
     r.half = sw && sw->half;
-    r.fp64_tiles = s.p.pcg_mode == 2;
+    r.fp64_tiles = s.p.pcg_mode == 2 || (sw && sw->max_m <= 32);
     r.sms = s.ctx->sm_count;
     r.nv = s.nv;
     r.ninst = K;

@@ -93,6 +93,23 @@ def test_random_patterns(ctx, nv):
         assert np.linalg.norm(r) / np.linalg.norm(b) <= 5e-6
 
 
+@pytest.mark.parametrize("n,domain", [(40, 1), (40, 8), (40, 10), (100, 8), (120, 10)])
+def test_one_tile_domains_sum_in_fp64(ctx, n, domain):
+    """The default mode over domains of one tile: as pcg_mode 2 above, against the one-warp fused kernel."""
+    sc = scenes.sheet_on_sphere(n, height=2.0)
+    sc["velocities"] = (60 * np.random.default_rng(n).standard_normal(sc["positions"].shape)).astype(np.float32)
+    out = []
+    for kw in (dict(pcg_variant=1), {}):
+        p = dict(sc["params"], self_collision=0, newton_iters=1, cg_max_iter=4, cg_tol=1e-9, schwarz_domain=domain, **kw)
+        g = ImplicitSolver(ctx, dict(sc, params=p), "mixed")
+        assert g.step(1)[0]["status"] == 0
+        out.append(g.positions.copy())
+        if not kw:
+            assert g.pcg_kernels() == (-1, -1)  # resident
+        g.close()
+    assert (out[0] == out[1]).mean() >= 0.999
+
+
 def test_solvers_on_threads_share_the_gpu():
     """Three threads, each with its own context and solver, solve at once: every launch wants all SMs, so
     they take turns, and each solution is the one a solver alone finds, bit for bit."""
