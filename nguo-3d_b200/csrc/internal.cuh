@@ -215,11 +215,21 @@ struct RsRun {
   // how many of a CTA's blocks may have no place packed before the solve is left to the other PCG
   // (resident_walked)
   uint32_t walked_max = 0;
+  uint32_t dom_max = 0xffffffffu;  // the most Schwarz domains a CTA may have for it, likewise
   uint32_t vert[PCG_MAX_INST + 1] = {}, dom[PCG_MAX_INST + 1] = {}, diag[PCG_MAX_INST] = {};
 };
 
 // walked_max: see resident_walked
 constexpr uint32_t WALKED_SCENE = 1500;
+// dom_max: a domain takes a team's turn whatever its size, 1.0 to 1.7 us over six teams' (three warps
+// each), so many small ones to a CTA lose to kernels that give each a warp anywhere on the chip. us an
+// iteration, resident and the other PCG (in brackets: domains a CTA):
+//   scenes, mixed: 150 x 150 sheet, domains of 16 (10) 17, 22, of 10 (16) 29, 22, of 8 (20) 35, 27; four
+//     coarse garments, 60 000 vertices in all, of 10 (17) 29, 33, of 8 (21) 35, 36;
+//   solver, mixed: 150 x 150 grid, of 8 (20) 28, 31, of 4 (39) 40, 39; 220 x 220, of 16 (21) 29, 40, of 8 (42)
+//     51, 42; 300 x 300, of 24 (26) 46, 69, of 16 (39) 64, 54, of 12 (52) 87, 68.
+inline uint32_t dom_max_scene(uint32_t nv) { return 11 + nv / 8000; }
+inline uint32_t dom_max_solver(uint32_t nv) { return 16 + nv / 4300; }
 inline uint32_t walked_solver(bool schwarz, uint32_t nv) { return schwarz ? 2800 + nv / 42 : 12000; }
 
 struct RsWork {

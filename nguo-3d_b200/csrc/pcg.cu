@@ -243,6 +243,7 @@ static int pcg_solve_resident(mguso_linear_solver* s, float tol, uint32_t max_it
     r.nv = a->nb;
     r.nnz = a->nnzb;
     r.walked_max = walked_solver(sw != nullptr, a->nb);
+    r.dom_max = dom_max_solver(a->nb);
     s->rs.good[0] = s->rs.poor[0] = 0;
     r.vert[1] = a->nb;
     if (sw && !resident_domains(*sw, r)) return MGUSO_ERR_UNSUPPORTED;

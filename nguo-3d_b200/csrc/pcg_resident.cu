@@ -1374,7 +1374,7 @@ int pcg_resident(const RsSystem& sys, const mguso_bsr& bsr, const mguso_schwarz*
     const uint32_t dom = ceil_div(nd[i], I.ncta), dia = 32 * ceil_div(I.dd1 - I.dd0, I.ncta);
     // the vectors of a CTA's vertices, the halo and the hash table have to fit
     const uint64_t need = RS_SCRATCH + 52ull * 32 * dom + 20ull * RS_MAX_HALO + 52ull * dia + 64 + RS_HASH_BYTES;
-    if (dom > (uint32_t)RS_MAX_DOM || need > smem) return MGUSO_ERR_UNSUPPORTED;
+    if (dom > (uint32_t)RS_MAX_DOM || need > smem || (sw && dom > run.dom_max)) return MGUSO_ERR_UNSUPPORTED;
     // looked at row by row, once: more CTAs fit at least as well
     const uint32_t stage = 2 * (RS_WARPS / (wide ? 6 : 3)) * RS_CHUNK;
     if (w.good[I.k] && I.ncta >= w.good[I.k]) continue;
@@ -1444,6 +1444,7 @@ int pcg_resident_scene(Scene& s, uint32_t active) {
     r.ninst = K;
     r.nnz = s.Ps.nnz;
     r.walked_max = WALKED_SCENE;
+    r.dom_max = dom_max_scene(s.nv);
     for (uint32_t k = 0; k <= K; ++k) r.vert[k] = s.inst_vert[k];
     MG_CHECK_ARG(!sw || resident_domains(*sw, r), "resident PCG: Schwarz domains are not grouped by instance");
     s.rs_ready = true;

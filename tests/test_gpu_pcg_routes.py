@@ -29,11 +29,12 @@ def test_solver_around_the_limit(ctx, n, precond):
         assert np.linalg.norm(r) / np.linalg.norm(b) <= 5e-6
 
 
-@pytest.mark.parametrize("n,precond,fused", [(300, 1, False), (360, 1, True), (330, 2, False), (400, 2, True)])
-def test_scenes_take_the_fused_kernels_where_rows_would_be_walked(ctx, n, precond, fused):
-    """20 and 28 runs a CTA (block Jacobi), 24 and 34 domains (Schwarz)."""
+@pytest.mark.parametrize("n,precond,domain,fused", [(300, 1, 32, False), (360, 1, 32, True), (330, 2, 32, False),
+                                                    (400, 2, 32, True), (100, 2, 8, False), (150, 2, 8, True)])
+def test_scenes_take_the_fused_kernels_where_rows_would_be_walked(ctx, n, precond, domain, fused):
+    """20 and 28 runs a CTA (block Jacobi), 24 and 34 domains (Schwarz); of small domains 9 and 20."""
     sc = scenes.sheet_on_sphere(n, height=0.32)
-    sc["params"] = dict(sc["params"], precond=precond, newton_iters=2)
+    sc["params"] = dict(sc["params"], precond=precond, schwarz_domain=domain, newton_iters=2)
     g = ImplicitSolver(ctx, sc, "mixed")
     assert g.step(1)[0]["status"] == 0
     assert (g.pcg_kernels() != (-1, -1)) == fused
